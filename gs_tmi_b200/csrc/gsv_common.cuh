@@ -135,6 +135,22 @@ __device__ __forceinline__ float4 tight_extent(const float qc[6]) {
                        __double2float_ru(sqrt(f * s2) + 0.01), 0.f);
 }
 
+// Threshold of the separating-plane test of a block (plane_separates in gsv_render.cu): 9.1, or
+// infinity (nothing is separated) where rounding could decide it.  The test is run in FP32 on the
+// stored coefficients; with K = max_a Q_aa S_aa <= 250 and sum_a sqrt(Q_aa) <= 800 its relative
+// errors stay below 2e-3 (m) and 0.014 sqrt(m) (t), and the row form's m is within 8.3e-4 of the exact
+// one: 0.99, 1.515 and 9.1 leave at least as much again.  K <= 1 / det(C) for the correlation matrix C of Q
+// (a cofactor of C is at most 1), and det(C) is computed here to about 1e-6.
+__device__ __forceinline__ float plane_threshold(const Rec& r) {
+    const float h01 = 0.5f * r.q01x2, h02 = 0.5f * r.q02x2, h12 = 0.5f * r.q12x2;
+    const float i0 = 1.0f / r.q00, i1 = 1.0f / r.q11, i2 = 1.0f / r.q22;
+    const float r01 = h01 * h01 * i0 * i1, r02 = h02 * h02 * i0 * i2, r12 = h12 * h12 * i1 * i2;
+    const float det = 1.0f + 2.0f * (h01 * i0) * (h02 * i2) * (h12 * i1) - r01 - r02 - r12;
+    const bool ok = r.q00 > 0.0f && r.q11 > 0.0f && r.q22 > 0.0f && r.q00 < 7e4f && r.q11 < 7e4f && r.q22 < 7e4f &&
+                    r01 < 1.0f && r02 < 1.0f && r12 < 1.0f && det >= 1.0f / 250.0f;
+    return ok ? 9.1f : __int_as_float(0x7f800000);
+}
+
 // Row terms of the quadratic form for fixed (e0, e1):
 //   m(e2) = fma(fma(q22, e2, B), e2, A)
 __device__ __forceinline__ float row_a(const Rec& g, float e0, float e1) {

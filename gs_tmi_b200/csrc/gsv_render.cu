@@ -1,6 +1,6 @@
 // gsv_render.cu -- forward / backward tile kernels and the gradient finalize.
 //
-// Work decomposition (tile edge 8, the reference default):
+// Forward, tile edge 8 (the reference default):
 //   one CTA of 4 warps per tile; every warp covers the whole 8x8x8 tile
 //   (lane l owns the two 8-voxel rows (d0+l/8, h0+l%8) and (d0+4+l/8, h0+l%8))
 //   and the tile's Gaussian list is dealt out to the warps position by
@@ -10,13 +10,14 @@
 //   each Gaussian a lane evaluates its 16 voxels with the row form
 //   m = fma(fma(q22, e2, B), e2, A) (A, B once per row), and the exp / FMA
 //   part runs only when some lane of the warp is inside the 3-sigma cutoff.
-//   Forward: per-warp partial tiles are summed through shared memory once
-//   per tile and stored as complex64.  Backward: per (tile, Gaussian) a
-//   lane folds its voxels into 11 moments, the warp reduce-scatters them
-//   (16 shuffles) and lanes issue one atomic per moment (or, deterministic,
-//   write the per-pair partial for a fixed-order reduction in finalize).
+//   The per-warp partial tiles are summed through shared memory once
+//   per tile and stored as complex64.
 //
-// Other tile edges use a generic one-voxel-per-thread kernel pair.
+// Backward, tile edge 8: one lane per (Gaussian, 4x4x4 block of the tile),
+//   see backward_tile.
+//
+// Other tile edges: 4 has kernels of its own (one warp per tile), the rest a
+// generic one-voxel-per-thread pair.
 //
 // Reference semantics (3DGS/3dgsVC/gaussian/cuda_ext/tile_voxelize_cuda_kernel.cu):
 //   forward  :118-141  vol = sum_{g in list(tile), m <= 9} exp(-m/2) rho_g
@@ -456,148 +457,351 @@ __global__ void __launch_bounds__(kThreads) k_forward8(const RenderArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Tile edge 8: backward
+// 4x4x4 blocks: the unit the render kernels evaluate
 // ---------------------------------------------------------------------------
 
-// Backward of one tile (RPL = 2) or half tile (RPL = 1); warp-synchronous
-// only.  The deterministic mode writes one partial per (tile, Gaussian) and
-// therefore runs with RPL = 2 only.
-template <bool COMPAT, bool DET, int RPL>
-__device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile, int sub, WarpStage* stage,
-                                              int part) {
-    static_assert(!DET || RPL == 2, "deterministic partials need the whole tile in one CTA");
-    constexpr int NV = RPL * 8;
-    const int2 rg = a.ranges[tile];
-    if (rg.x >= rg.y) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int d0, h0, w0;
-    decode_tile(a, tile, d0, h0, w0);
-    float ih[3];
-    compat_ih<COMPAT>(a, ih);
-    const int chunk = a.chunk;
+constexpr int kBlk = 4;                     // edge of a block
+constexpr int kBlkVox = kBlk * kBlk * kBlk;
+// Above this magnitude a density or an upstream gradient may overflow a product that a voxel outside
+// the cutoff must not see; such inputs (and NaN) take the guarded loop.
+constexpr float kBig = 1e15f;
 
-    // Upstream gradient of the lane's voxels (zero outside the volume).
-    float gr[NV], gi[NV];
-    {
-        const int gh = h0 + (lane & 7);
+__device__ __forceinline__ float4 rec_quad(const Rec& r, int i) {
+    return i == 0 ? make_float4(r.c0, r.c1, r.c2, r.q00)
+                  : (i == 1 ? make_float4(r.q01x2, r.q02x2, r.q11, r.q12x2) : make_float4(r.q22, r.rho_r, r.rho_i, 0.f));
+}
+__device__ __forceinline__ Rec rec_of(float4 x, float4 y, float4 z) {
+    Rec r;
+    r.c0 = x.x; r.c1 = x.y; r.c2 = x.z; r.q00 = x.w;
+    r.q01x2 = y.x; r.q02x2 = y.y; r.q11 = y.z; r.q12x2 = y.w;
+    r.q22 = z.x; r.rho_r = z.y; r.rho_i = z.z; r.pad = 0.0f;
+    return r;
+}
+
+// Separating plane of a Gaussian's inclusion set and a block, from the block centre's offset e to the
+// Gaussian: with n = Q e (the gradient there, up to a factor), the block's voxels x satisfy
+// n.x >= m(e) - 1.5 |n|_1, and {m <= 9} lies in n.x <= 3 sqrt(m(e)).  `thr`: plane_threshold.  On
+// fits' Gaussians 93-96% of the blocks kept by this test and the extent hold an included voxel;
+// the extent's box alone keeps 1.4 to 1.6 times as many.
+__device__ __forceinline__ bool plane_separates(float n0, float n1, float n2, float e0, float e1, float e2, float thr) {
+    const float m = fmaf(n0, e0, fmaf(n1, e1, n2 * e2));
+    const float t = fmaf(-1.515f, fabsf(n0) + fabsf(n1) + fabsf(n2), 0.99f * m);
+    return t > 0.0f && t * t > thr * m;
+}
+
+// Which of a tile's eight blocks (bit 4 bd + 2 bh + bw) may hold a voxel the Gaussian includes.
+// x: its tight extent (w: the plane threshold); without `use_box` only the planes are tried.
+__device__ __forceinline__ unsigned block_mask8(const Rec& r, float4 x, int d0, int h0, int w0, bool use_box) {
+    unsigned in = 0xff;
+    if (use_box) {
+        const float lo0 = __fsub_rn(r.c0, x.x), hi0 = __fadd_rn(r.c0, x.x);
+        const float lo1 = __fsub_rn(r.c1, x.y), hi1 = __fadd_rn(r.c1, x.y);
+        const float lo2 = __fsub_rn(r.c2, x.z), hi2 = __fadd_rn(r.c2, x.z);
+        in = ((lo0 <= float(d0 + 3) && hi0 >= float(d0)) ? 0x0fu : 0u) |
+             ((lo0 <= float(d0 + 7) && hi0 >= float(d0 + 4)) ? 0xf0u : 0u);
+        in &= ((lo1 <= float(h0 + 3) && hi1 >= float(h0)) ? 0x33u : 0u) |
+              ((lo1 <= float(h0 + 7) && hi1 >= float(h0 + 4)) ? 0xccu : 0u);
+        in &= ((lo2 <= float(w0 + 3) && hi2 >= float(w0)) ? 0x55u : 0u) |
+              ((lo2 <= float(w0 + 7) && hi2 >= float(w0 + 4)) ? 0xaau : 0u);
+    }
+    const float thr = x.w;
+    const float h01 = 0.5f * r.q01x2, h02 = 0.5f * r.q02x2, h12 = 0.5f * r.q12x2;
 #pragma unroll
-        for (int r = 0; r < RPL; ++r) {
-            const int gd = d0 + (lane >> 3) + 4 * (r + sub);
-            const bool row_ok = gd < a.d && gh < a.h;
-            const int64_t flat = (int64_t(gd) * a.h + gh) * a.w + w0;
+    for (int bd = 0; bd < 2; ++bd) {
+        const float e0 = float(d0 + 4 * bd) + 1.5f - r.c0;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const bool ok = row_ok && (w0 + k < a.w);
-                if (COMPAT) {
-                    gr[r * 8 + k] = ok ? __ldg(a.gv_r + flat + k) : 0.0f;
-                    gi[r * 8 + k] = ok ? __ldg(a.gv_i + flat + k) : 0.0f;
-                } else {
-                    const float2 x = ok ? __ldg(reinterpret_cast<const float2*>(a.gvol) + flat + k)
-                                        : make_float2(0.f, 0.f);
-                    gr[r * 8 + k] = x.x;
-                    gi[r * 8 + k] = x.y;
-                }
+        for (int bh = 0; bh < 2; ++bh) {
+            const float e1 = float(h0 + 4 * bh) + 1.5f - r.c1;
+            const float a0 = fmaf(h01, e1, r.q00 * e0), a1 = fmaf(h01, e0, r.q11 * e1), a2 = fmaf(h02, e0, h12 * e1);
+#pragma unroll
+            for (int bw = 0; bw < 2; ++bw) {
+                const float e2 = float(w0 + 4 * bw) + 1.5f - r.c2;
+                if (plane_separates(fmaf(h02, e2, a0), fmaf(h12, e2, a1), fmaf(r.q22, e2, a2), e0, e1, e2, thr))
+                    in &= ~(1u << (4 * bd + 2 * bh + bw));
             }
         }
     }
+    return in;
+}
 
-    float ev0[RPL];
+// One Gaussian's 11 moments over one block, all in one lane.  gs: the block's upstream gradient,
+// (re, im) by (d, h, w); v0..v2: the block's first voxel.  The weight of an excluded voxel is zero;
+// GUARD excludes such voxels from every product instead (infinite, NaN or huge inputs) and returns
+// zeros when no voxel is included.
+template <bool GUARD>
+__device__ __forceinline__ void block_moments(const Rec& g, const float2* gs, float v0, float v1, float v2,
+                                              float mom[kMomStride]) {
+    float e1[kBlk], e1s[kBlk], qe[kBlk], e2[kBlk], e2s[kBlk];
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) ev0[r] = float(d0 + (lane >> 3) + 4 * (r + sub));
-    const float ev1 = float(h0 + (lane & 7));
-    WarpStage& S = stage[warp];
+    for (int k = 0; k < kBlk; ++k) {
+        e1[k] = __fsub_rn(v1 + float(k), g.c1);
+        e1s[k] = e1[k] * e1[k];
+        qe[k] = __fmul_rn(__fmul_rn(g.q11, e1[k]), e1[k]);
+        e2[k] = __fsub_rn(v2 + float(k), g.c2);
+        e2s[k] = e2[k] * e2[k];
+    }
+    const float hr = -0.5f * g.rho_r, hi = -0.5f * g.rho_i;
+    float Dr = 0.f, Di = 0.f, S0 = 0.f, S1 = 0.f, S2 = 0.f;
+    float M00 = 0.f, M01 = 0.f, M02 = 0.f, M11 = 0.f, M12 = 0.f, M22 = 0.f;
+    bool any = false;
+#pragma unroll 1
+    for (int i = 0; i < kBlk; ++i) {
+        const float e0 = __fsub_rn(v0 + float(i), g.c0);
+        const float q0e = __fmul_rn(g.q00, e0), qb = __fmul_rn(g.q02x2, e0);
+        // the plane's sums (of w g_r, w g_i, a, a e1, a e2, a e1^2, a e1 e2, a e2^2): summed by planes so that
+        // no chain is long
+        float Pr = 0.f, Pi = 0.f, P0 = 0.f, P1 = 0.f, P2 = 0.f, P11 = 0.f, P12 = 0.f, P22 = 0.f;
+#pragma unroll
+        for (int j = 0; j < kBlk; ++j) {
+            // row_a, row_b
+            const float A = __fmaf_rn(__fmaf_rn(g.q01x2, e1[j], q0e), e0, qe[j]);
+            const float B = __fmaf_rn(g.q12x2, e1[j], qb);
+            const float4* row = reinterpret_cast<const float4*>(gs + (i * kBlk + j) * kBlk);
+            const float4 ga = row[0], gb = row[1];
+            const float gr[kBlk] = {ga.x, ga.z, gb.x, gb.z}, gi[kBlk] = {ga.y, ga.w, gb.y, gb.w};
+            float R0 = 0.f, R1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < kBlk; ++k) {
+                const float m = row_m(g.q22, A, B, e2[k]);
+                const bool in = m <= kCut;
+                if (GUARD) {
+                    if (in) {
+                        const float w = ex2_approx(m * kNegHalfLog2e);
+                        const float a = w * fmaf(hi, gi[k], hr * gr[k]);
+                        Pr = fmaf(w, gr[k], Pr);
+                        Pi = fmaf(w, gi[k], Pi);
+                        R0 += a;
+                        R1 = fmaf(a, e2[k], R1);
+                        P22 = fmaf(a, e2s[k], P22);
+                        any = true;
+                    }
+                } else {
+                    const float x = ex2_approx(m * kNegHalfLog2e);
+                    const float w = in ? x : 0.f;
+                    const float a = w * fmaf(hi, gi[k], hr * gr[k]);
+                    Pr = fmaf(w, gr[k], Pr);
+                    Pi = fmaf(w, gi[k], Pi);
+                    R0 += a;
+                    R1 = fmaf(a, e2[k], R1);
+                    P22 = fmaf(a, e2s[k], P22);
+                }
+            }
+            P0 += R0;
+            P1 = fmaf(e1[j], R0, P1);
+            P2 += R1;
+            P11 = fmaf(e1s[j], R0, P11);
+            P12 = fmaf(e1[j], R1, P12);
+        }
+        const float u = e0 * P0;
+        Dr += Pr;
+        Di += Pi;
+        M11 += P11;
+        M12 += P12;
+        M22 += P22;
+        S0 += u;
+        S1 += P1;
+        S2 += P2;
+        M00 = fmaf(e0, u, M00);
+        M01 = fmaf(e0, P1, M01);
+        M02 = fmaf(e0, P2, M02);
+    }
+    mom[0] = Dr; mom[1] = Di; mom[2] = S0; mom[3] = S1; mom[4] = S2;
+    mom[5] = M00; mom[6] = M01; mom[7] = M02; mom[8] = M11; mom[9] = M12; mom[10] = M22; mom[11] = 0.f;
+    if (GUARD && !any) {
+#pragma unroll
+        for (int i = 0; i < kMomStride; ++i) mom[i] = 0.f;
+    }
+}
+
+// Whether a Gaussian needs the guarded loop of block_moments.
+__device__ __forceinline__ bool needs_guard(const Rec& r) {
+    return !(fabsf(r.rho_r) <= kBig && fabsf(r.rho_i) <= kBig && fabsf(r.c0) <= kBig && fabsf(r.c1) <= kBig &&
+             fabsf(r.c2) <= kBig);
+}
+
+// The moments of one (tile, Gaussian) pair to the gradients of the reference's own parameters.
+__device__ __forceinline__ void compat_emit_lane(const RenderArgs& a, const Rec& g, int gid, const float m[kMomStride],
+                                                 const float ih[3]) {
+    atomicAdd(a.g_dr + gid, m[0]);
+    atomicAdd(a.g_di + gid, m[1]);
+    // dL/dcenter_a = -2 sum_b Q_ab S1_b   (reference: -2 (M d)_a / hs_a, .cu:241-243)
+    float* gc = a.g_center + int64_t(gid) * 3;
+    atomicAdd(gc, -(2.0f * g.q00 * m[2] + g.q01x2 * m[3] + g.q02x2 * m[4]));
+    atomicAdd(gc + 1, -(g.q01x2 * m[2] + 2.0f * g.q11 * m[3] + g.q12x2 * m[4]));
+    atomicAdd(gc + 2, -(g.q02x2 * m[2] + g.q12x2 * m[3] + 2.0f * g.q22 * m[4]));
+    // dL/dcov_inv_ab = sum a d_a d_b = S2_ab / (hs_a hs_b)  (.cu:244-252)
+    float* gm = a.g_cov + int64_t(gid) * 9;
+    const float c01 = m[6] * ih[0] * ih[1], c02 = m[7] * ih[0] * ih[2], c12 = m[9] * ih[1] * ih[2];
+    atomicAdd(gm, m[5] * ih[0] * ih[0]);
+    atomicAdd(gm + 1, c01);
+    atomicAdd(gm + 2, c02);
+    atomicAdd(gm + 3, c01);
+    atomicAdd(gm + 4, m[8] * ih[1] * ih[1]);
+    atomicAdd(gm + 5, c12);
+    atomicAdd(gm + 6, c02);
+    atomicAdd(gm + 7, c12);
+    atomicAdd(gm + 8, m[10] * ih[2] * ih[2]);
+}
+
+// ---------------------------------------------------------------------------
+// Tile edge 8: backward
+// ---------------------------------------------------------------------------
+
+// One lane per (Gaussian, 4^3 block): the lane walks the block's 64 voxels and keeps the Gaussian's
+// moments to itself, so nothing is reduced across lanes.  (The kernel before it had a warp's lanes
+// share one Gaussian over 4x8x8 voxels: 13 shuffles and as many selects per pair, and 16 voxels per
+// lane of which 11-25% were inside the cutoff; the blocks kept here are 23-45% inside.)  A warp stages
+// up to kBwdCap kept Gaussians of its share of the tile's list, lists their (Gaussian, block) tasks
+// block by block, and deals the tasks to its lanes 32 at a time; a Gaussian's tasks add up in shared
+// memory in block order, so its pair total does not depend on which lanes ran them.
+constexpr int kBwdCap = 64;
+constexpr int kGradStride = kBlkVox + 2;  // float2 per block of the staged gradient: two blocks' rows in other banks
+
+struct __align__(16) BwdStage {
+    float4 rec[kBwdCap][3];
+    float4 mom[kBwdCap][3];
+    int32_t gid[kBwdCap];
+    int32_t pidx[kBwdCap];          // deterministic: emission index of the pair
+    uint16_t task[kBwdCap * 8];     // Gaussian slot | block << 8, by block
+    uint8_t mask[kBwdCap];
+};
+
+// Backward of one tile (RPL = 2) or of its half `sub` (RPL = 1).  One CTA barrier.
+template <bool COMPAT, bool DET, int RPL>
+__device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile, int sub, BwdStage* stage,
+                                              float2* grad, int part) {
+    static_assert(!DET || RPL == 2, "deterministic partials need the whole tile in one CTA");
+    const int2 rg = a.ranges[tile];
+    if (rg.x >= rg.y) return;  // CTA-uniform
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int d0, h0, w0;
+    decode_tile(a, tile, d0, h0, w0);
+
+    // The tile's upstream gradient, by block (zero outside the volume): thread t takes half a row.
+    bool guard = false;
+    {
+        const int row = threadIdx.x >> 1, bw = threadIdx.x & 1;
+        const int ld = row >> 3, lh = row & 7;
+        const int gd = d0 + ld, gh = h0 + lh, gw = w0 + kBlk * bw;
+        const bool row_ok = gd < a.d && gh < a.h;
+        const int64_t flat = (int64_t(gd) * a.h + gh) * a.w + gw;
+        const int blk = (ld >> 2) * 4 + (lh >> 2) * 2 + bw;
+        float2* dst = grad + blk * kGradStride + ((ld & 3) * kBlk + (lh & 3)) * kBlk;
+#pragma unroll
+        for (int k = 0; k < kBlk; ++k) {
+            float2 x = make_float2(0.f, 0.f);
+            if (row_ok && gw + k < a.w)
+                x = COMPAT ? make_float2(__ldg(a.gv_r + flat + k), __ldg(a.gv_i + flat + k))
+                           : __ldg(reinterpret_cast<const float2*>(a.gvol) + flat + k);
+            guard |= !(fabsf(x.x) <= kBig && fabsf(x.y) <= kBig);
+            dst[k] = x;
+        }
+    }
+    guard = __syncthreads_or(guard);
+
+    float ih[3];
+    compat_ih<COMPAT>(a, ih);
+    BwdStage& S = stage[warp];
     // list positions of this warp: first, first + stride, ... (part `part` of a.split CTAs)
     const int stride = kWarps * a.split, first = part * kWarps + warp;
     const int mine = rg.y - rg.x > first ? (rg.y - rg.x - first + stride - 1) / stride : 0;
-    for (int i0 = 0; i0 < mine; i0 += chunk) {
-        const int base = rg.x + first + stride * i0;
-        const int kept =
-            stage_chunk<COMPAT, RPL, DET>(a, S, base, stride, min(chunk, mine - i0), lane, d0, h0, w0, sub, ih);
-        __syncwarp();
-        for (int j = 0; j < kept; ++j) {
-            const Rec g = S.rec[j];
-            const int bits = S.meta[j];  // warp-uniform
-            const float4 ea = S.e2[j][0], eb = S.e2[j][1];
-            const float e2[8] = {ea.x, ea.y, ea.z, ea.w, eb.x, eb.y, eb.z, eb.w};
-            const float e1 = __fsub_rn(ev1, g.c1);
-            const float hr = -0.5f * g.rho_r, hi = -0.5f * g.rho_i;
-            // per row: Dr/Di = sum w g_r / g_i; R1/R2 = sum a e2 / a e2^2 with
-            // a = w (hr g_r + hi g_i); sum a itself = hr Dr + hi Di (after the loop)
-            float e0[RPL], Dr[RPL], Di[RPL], R1[RPL], R2[RPL];
-            bool wany = false;
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) {
-                e0[r] = __fsub_rn(ev0[r], g.c0);
-                Dr[r] = Di[r] = R1[r] = R2[r] = 0.f;
-                if (!(bits & (1 << r))) continue;  // slot out of the Gaussian's extent
-                const float A = row_a(g, e0[r], e1), B = row_b(g, e0[r], e1);
-                float m[8];
-                bool any = false;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    m[k] = row_m(g.q22, A, B, e2[k]);
-                    any |= (m[k] <= kCut);
+    const unsigned blocks = RPL == 2 ? 0xffu : 0xfu << (4 * sub);
+    for (int i0 = 0; i0 < mine;) {
+        int kept = 0;
+        for (; i0 < mine && kept + a.chunk <= kBwdCap; i0 += a.chunk) {
+            Rec r;
+            int gid = 0;
+            unsigned in = 0;
+            const bool listed = lane < min(a.chunk, mine - i0);
+            if (listed) {
+                gid = __ldg(a.pair_ids + rg.x + first + stride * (i0 + lane));
+                r = load_rec<COMPAT>(a, gid, ih);
+                in = blocks;
+                if (a.cull) {
+                    const float4 x = COMPAT ? make_float4(0.f, 0.f, 0.f, plane_threshold(r)) : __ldg(a.ext + gid);
+                    in &= block_mask8(r, x, d0, h0, w0, !COMPAT);
                 }
-                if (!__any_sync(kFull, any)) continue;  // warp-uniform row-slot skip
-                wany = true;
+            }
+            const unsigned keep = __ballot_sync(kFull, in != 0);
+            if (DET && listed && !in) {  // dropped pair: its partial is zero
+                float4* dst = reinterpret_cast<float4*>(a.partials +
+                                                        emission_index(a, gid, d0 >> 3, h0 >> 3, w0 >> 3) * kMomStride);
+                dst[0] = dst[1] = dst[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if (in) {
+                const int pos = kept + __popc(keep & ((1u << lane) - 1u));
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int q = r * 8 + k;
-                    if (m[k] <= kCut) {
-                        const float wgt = ex2_approx(m[k] * kNegHalfLog2e);
-                        Dr[r] = fmaf(wgt, gr[q], Dr[r]);
-                        Di[r] = fmaf(wgt, gi[q], Di[r]);
-                        const float ae = wgt * fmaf(hi, gi[q], hr * gr[q]) * e2[k];
-                        R1[r] += ae;
-                        R2[r] = fmaf(ae, e2[k], R2[r]);
+                for (int i = 0; i < 3; ++i) {
+                    S.rec[pos][i] = rec_quad(r, i);
+                    S.mom[pos][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                S.gid[pos] = gid;
+                S.mask[pos] = uint8_t(in);
+                if (DET) S.pidx[pos] = int32_t(emission_index(a, gid, d0 >> 3, h0 >> 3, w0 >> 3));
+            }
+            kept += __popc(keep);
+        }
+        __syncwarp();
+        // tasks, block by block, each block's Gaussians in list order
+        int tasks = 0;
+        unsigned m0 = lane < kept ? S.mask[lane] : 0u, m1 = lane + 32 < kept ? S.mask[lane + 32] : 0u;
+        static_assert(kBwdCap == 64, "two mask words per lane");
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const bool hit = ((s ? m1 : m0) >> b) & 1u;
+                const unsigned bal = __ballot_sync(kFull, hit);
+                if (hit) S.task[tasks + __popc(bal & ((1u << lane) - 1u))] = uint16_t((lane + 32 * s) | (b << 8));
+                tasks += __popc(bal);
+            }
+        }
+        __syncwarp();
+        for (int t0 = 0; t0 < tasks; t0 += 32) {
+            const bool on = t0 + lane < tasks;
+            const unsigned task = S.task[on ? t0 + lane : tasks - 1];
+            const int slot = task & 0xff, b = task >> 8;
+            const Rec g = rec_of(S.rec[slot][0], S.rec[slot][1], S.rec[slot][2]);
+            const float2* gs = grad + b * kGradStride;
+            const float v0 = float(d0 + (b >> 2) * kBlk), v1 = float(h0 + ((b >> 1) & 1) * kBlk),
+                        v2 = float(w0 + (b & 1) * kBlk);
+            float m[kMomStride];
+            if (guard || __any_sync(kFull, needs_guard(g))) block_moments<true>(g, gs, v0, v1, v2, m);
+            else block_moments<false>(g, gs, v0, v1, v2, m);
+            // a Gaussian may have two of its blocks among these lanes: one block at a time
+            const int b_end = __shfl_sync(kFull, b, 31);
+            for (int bb = __shfl_sync(kFull, b, 0); bb <= b_end; ++bb) {
+                if (on && b == bb) {
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        float4 x = S.mom[slot][i];
+                        x.x += m[4 * i];
+                        x.y += m[4 * i + 1];
+                        x.z += m[4 * i + 2];
+                        x.w += m[4 * i + 3];
+                        S.mom[slot][i] = x;
                     }
                 }
+                __syncwarp();
             }
-            if (!wany) {  // no included voxel here: the pair's partial is zero
-                if (DET && lane == 0) {
-                    float4* dst = reinterpret_cast<float4*>(a.partials + int64_t(S.pidx[j]) * kMomStride);
-                    dst[0] = dst[1] = dst[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                continue;
-            }
-            float v[16];
-            float Drs = 0.f, Dis = 0.f, R0s = 0.f, R1s = 0.f, R2s = 0.f, S1 = 0.f, S2 = 0.f, S3 = 0.f;
-            float R0[RPL];
-#pragma unroll
-            for (int r = 0; r < RPL; ++r) {
-                R0[r] = fmaf(hi, Di[r], hr * Dr[r]);
-                Drs += Dr[r];
-                Dis += Di[r];
-                R0s += R0[r];
-                R1s += R1[r];
-                R2s += R2[r];
-                S1 = fmaf(e0[r], R0[r], S1);          // sum a e0
-                S2 = fmaf(e0[r] * e0[r], R0[r], S2);  // sum a e0^2
-                S3 = fmaf(e0[r], R1[r], S3);          // sum a e0 e2
-            }
-            v[0] = Drs;
-            v[1] = Dis;
-            v[2] = S1;
-            v[3] = e1 * R0s;
-            v[4] = R1s;
-            v[5] = S2;
-            v[6] = e1 * S1;
-            v[7] = S3;
-            v[8] = (e1 * e1) * R0s;
-            v[9] = e1 * R1s;
-            v[10] = R2s;
-            const int gid = S.gid[j];
+        }
+        for (int k = lane; k < kept; k += 32) {
+            const int gid = S.gid[k];
             if (COMPAT) {
+                float m[kMomStride];
 #pragma unroll
-                for (int i = 11; i < 16; ++i) v[i] = 0.f;
-                compat_emit(a, g, gid, warp_reduce_scatter16(v, lane), lane, ih);
+                for (int i = 0; i < 3; ++i) {
+                    const float4 x = S.mom[k][i];
+                    m[4 * i] = x.x; m[4 * i + 1] = x.y; m[4 * i + 2] = x.z; m[4 * i + 3] = x.w;
+                }
+                compat_emit_lane(a, rec_of(S.rec[k][0], S.rec[k][1], S.rec[k][2]), gid, m, ih);
             } else {
-                v[11] = 0.f;
-                const float tot = warp_reduce_scatter12(v, lane);
-                const int mi = moment12(lane);
-                if (!(lane & 1) && mi >= 0 && mi < kMom) {
-                    if (DET) a.partials[int64_t(S.pidx[j]) * kMomStride + mi] = tot;
-                    else atomicAdd(a.accum + int64_t(gid) * kMomStride + mi, tot);
+                float4* dst = reinterpret_cast<float4*>(DET ? a.partials + int64_t(S.pidx[k]) * kMomStride
+                                                            : a.accum + int64_t(gid) * kMomStride);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    if (DET) dst[i] = S.mom[k][i];
+                    else atomicAdd(dst + i, S.mom[k][i]);
                 }
             }
         }
@@ -606,14 +810,12 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
 }
 
 template <bool COMPAT, bool DET, int RPL>
-// Register cap: 6 resident CTAs per SM for whole tiles (80 registers), 7 for
-// half tiles (72); a few spilled bytes outside the inner loop cost less
-// than the occupancy they buy (measured on B200).
-__global__ void __launch_bounds__(kThreads, RPL == 2 ? 6 : 7) k_backward8(const RenderArgs a) {
-    __shared__ __align__(16) WarpStage stage[kWarps];
+__global__ void __launch_bounds__(kThreads, 5) k_backward8(const RenderArgs a) {
+    __shared__ __align__(16) BwdStage stage[kWarps];
+    __shared__ __align__(16) float2 grad[8 * kGradStride];
     constexpr int subs = 2 / RPL;
     const int part = blockIdx.x % a.split, rest = blockIdx.x / a.split;
-    backward_tile<COMPAT, DET, RPL>(a, rest / subs, rest % subs, stage, part);
+    backward_tile<COMPAT, DET, RPL>(a, rest / subs, rest % subs, stage, grad, part);
 }
 
 // ---------------------------------------------------------------------------
@@ -1133,8 +1335,9 @@ __global__ void __launch_bounds__(kThreads) k_forward8_batched(const BatchTable 
 }
 
 template <bool DET>
-__global__ void __launch_bounds__(kThreads, 6) k_backward8_batched(const BatchTable t) {
-    __shared__ __align__(16) WarpStage stage[kWarps];
+__global__ void __launch_bounds__(kThreads, 5) k_backward8_batched(const BatchTable t) {
+    __shared__ __align__(16) BwdStage stage[kWarps];
+    __shared__ __align__(16) float2 grad[8 * kGradStride];
     __shared__ long long s_next;
     const int64_t total = t.tile_prefix[t.count];
     for (;;) {
@@ -1144,7 +1347,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_backward8_batched(const BatchTa
         const int64_t gt = s_next;
         if (gt >= total) break;
         const int i = find_item(t.tile_prefix, t.count, gt);
-        backward_tile<false, DET, 2>(t.items[i], gt - t.tile_prefix[i], 0, stage, 0);
+        backward_tile<false, DET, 2>(t.items[i], gt - t.tile_prefix[i], 0, stage, grad, 0);
     }
 }
 

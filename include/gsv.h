@@ -205,7 +205,7 @@ GSV_API int gsv_backward_batched(void* ws_batch, int count, int flags, void* str
 /* No counterpart in the reference.  rows_per_lane: 2 = one CTA per 8^3 tile
  * (two 8-voxel rows per lane), 1 = one CTA per 4x8x8 half tile (one row per
  * lane; the deterministic backward always uses whole tiles).  chunk: number
- * of Gaussians a warp stages in shared memory at a time (1..32).  flags:
+ * of list positions a warp stages in shared memory at a time (1..32).  flags:
  * GSV_TUNE_NO_CULL turns off the extent cull (a Gaussian, or a 4x8x8 row
  * slot of it, whose conservative tight extent misses the CTA's voxels is
  * skipped; it contributes nothing there either way).  split: the
