@@ -73,7 +73,8 @@ struct RenderArgs {
     float* g_di;
     int chunk;  // Gaussians staged per warp chunk (<= 32)
     int cull;   // skip Gaussians / row slots outside the tight extent
-    int split;  // backward: CTAs sharing one (half) tile's list, each taking every split-th quarter
+    int split;  // backward: CTAs that may share one (half) tile's list ...
+    int part;   // ... one for each started `part` positions
     // finalize
     gsv_params prm;
     gsv_grads grd;
@@ -524,96 +525,122 @@ __device__ __forceinline__ unsigned block_mask8(const Rec& r, float4 x, int d0, 
     return in;
 }
 
-// One Gaussian's 11 moments over one block, all in one lane.  gs: the block's upstream gradient,
-// (re, im) by (d, h, w); v0..v2: the block's first voxel.  The weight of an excluded voxel is zero;
-// GUARD excludes such voxels from every product instead (infinite, NaN or huge inputs) and returns
-// zeros when no voxel is included.
-template <bool GUARD>
-__device__ __forceinline__ void block_moments(const Rec& g, const float2* gs, float v0, float v1, float v2,
-                                              float mom[kMomStride]) {
-    float e1[kBlk], e1s[kBlk], qe[kBlk], e2[kBlk], e2s[kBlk];
-#pragma unroll
-    for (int k = 0; k < kBlk; ++k) {
-        e1[k] = __fsub_rn(v1 + float(k), g.c1);
-        e1s[k] = e1[k] * e1[k];
-        qe[k] = __fmul_rn(__fmul_rn(g.q11, e1[k]), e1[k]);
-        e2[k] = __fsub_rn(v2 + float(k), g.c2);
-        e2s[k] = e2[k] * e2[k];
-    }
-    const float hr = -0.5f * g.rho_r, hi = -0.5f * g.rho_i;
-    float Dr = 0.f, Di = 0.f, S0 = 0.f, S1 = 0.f, S2 = 0.f;
-    float M00 = 0.f, M01 = 0.f, M02 = 0.f, M11 = 0.f, M12 = 0.f, M22 = 0.f;
-    bool any = false;
-#pragma unroll 1
-    for (int i = 0; i < kBlk; ++i) {
-        const float e0 = __fsub_rn(v0 + float(i), g.c0);
-        const float q0e = __fmul_rn(g.q00, e0), qb = __fmul_rn(g.q02x2, e0);
-        // the plane's sums (of w g_r, w g_i, a, a e1, a e2, a e1^2, a e1 e2, a e2^2): summed by planes so that
-        // no chain is long
-        float Pr = 0.f, Pi = 0.f, P0 = 0.f, P1 = 0.f, P2 = 0.f, P11 = 0.f, P12 = 0.f, P22 = 0.f;
-#pragma unroll
-        for (int j = 0; j < kBlk; ++j) {
-            // row_a, row_b
-            const float A = __fmaf_rn(__fmaf_rn(g.q01x2, e1[j], q0e), e0, qe[j]);
-            const float B = __fmaf_rn(g.q12x2, e1[j], qb);
-            const float4* row = reinterpret_cast<const float4*>(gs + (i * kBlk + j) * kBlk);
-            const float4 ga = row[0], gb = row[1];
-            const float gr[kBlk] = {ga.x, ga.z, gb.x, gb.z}, gi[kBlk] = {ga.y, ga.w, gb.y, gb.w};
-            float R0 = 0.f, R1 = 0.f;
-#pragma unroll
-            for (int k = 0; k < kBlk; ++k) {
-                const float m = row_m(g.q22, A, B, e2[k]);
-                const bool in = m <= kCut;
-                if (GUARD) {
-                    if (in) {
-                        const float w = ex2_approx(m * kNegHalfLog2e);
-                        const float a = w * fmaf(hi, gi[k], hr * gr[k]);
-                        Pr = fmaf(w, gr[k], Pr);
-                        Pi = fmaf(w, gi[k], Pi);
-                        R0 += a;
-                        R1 = fmaf(a, e2[k], R1);
-                        P22 = fmaf(a, e2s[k], P22);
-                        any = true;
-                    }
-                } else {
-                    const float x = ex2_approx(m * kNegHalfLog2e);
-                    const float w = in ? x : 0.f;
-                    const float a = w * fmaf(hi, gi[k], hr * gr[k]);
-                    Pr = fmaf(w, gr[k], Pr);
-                    Pi = fmaf(w, gi[k], Pi);
-                    R0 += a;
-                    R1 = fmaf(a, e2[k], R1);
-                    P22 = fmaf(a, e2s[k], P22);
-                }
-            }
-            P0 += R0;
-            P1 = fmaf(e1[j], R0, P1);
-            P2 += R1;
-            P11 = fmaf(e1s[j], R0, P11);
-            P12 = fmaf(e1[j], R1, P12);
-        }
-        const float u = e0 * P0;
-        Dr += Pr;
-        Di += Pi;
-        M11 += P11;
-        M12 += P12;
-        M22 += P22;
-        S0 += u;
-        S1 += P1;
-        S2 += P2;
-        M00 = fmaf(e0, u, M00);
-        M01 = fmaf(e0, P1, M01);
-        M02 = fmaf(e0, P2, M02);
-    }
-    mom[0] = Dr; mom[1] = Di; mom[2] = S0; mom[3] = S1; mom[4] = S2;
-    mom[5] = M00; mom[6] = M01; mom[7] = M02; mom[8] = M11; mom[9] = M12; mom[10] = M22; mom[11] = 0.f;
-    if (GUARD && !any) {
-#pragma unroll
-        for (int i = 0; i < kMomStride; ++i) mom[i] = 0.f;
-    }
+// Packed pairs of FP32 (two rows of a block at once): each half rounds as the scalar operation does.
+typedef float2 f32x2;
+__device__ __forceinline__ f32x2 dup2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float sum2(f32x2 x) {
+    return x.x + x.y;
 }
 
-// Whether a Gaussian needs the guarded loop of block_moments.
+// The staged upstream gradient of a block: rows j, j + 1 (j even) of a plane side by side, one float4
+// {re j, re j+1, im j, im j+1} per voxel column.
+__device__ __forceinline__ int grad_at(int i, int j, int k) { return ((i * 2 + (j >> 1)) * kBlk + k) * 4 + (j & 1); }
+
+// One Gaussian's 11 moments over one block, all in one lane.  gs: the block's staged upstream gradient;
+// v0..v2: the block's first voxel.  The weight of an excluded voxel is zero.  Bound by FP32 issue:
+// packed pairs of rows take 39 issue slots per row of four voxels where the scalar form takes 66, and
+// the FMA pipe the same time.
+__device__ __forceinline__ void block_moments(const Rec& g, const float* gs, float v0, float v1, float v2,
+                                              float mom[kMomStride]) {
+    f32x2 e1[2], e1s[2], qe[2], e2[kBlk], e2s[kBlk];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const float lo = __fsub_rn(v1 + float(2 * p), g.c1), hi = __fsub_rn(v1 + float(2 * p + 1), g.c1);
+        e1[p] = make_float2(lo, hi);
+        e1s[p] = mul2(e1[p], e1[p]);
+        qe[p] = mul2(mul2(dup2(g.q11), e1[p]), e1[p]);
+    }
+#pragma unroll
+    for (int k = 0; k < kBlk; ++k) {
+        e2[k] = dup2(__fsub_rn(v2 + float(k), g.c2));
+        e2s[k] = mul2(e2[k], e2[k]);
+    }
+    const f32x2 hr = dup2(-0.5f * g.rho_r), hi = dup2(-0.5f * g.rho_i);
+    const f32x2 q01 = dup2(g.q01x2), q12 = dup2(g.q12x2), q22 = dup2(g.q22), scale = dup2(kNegHalfLog2e);
+    const f32x2 zero = dup2(0.f);
+    f32x2 Dr = zero, Di = zero, M11 = zero, M12 = zero, M22 = zero;
+    float S0 = 0.f, S1 = 0.f, S2 = 0.f, M00 = 0.f, M01 = 0.f, M02 = 0.f;
+#pragma unroll 2
+    for (int i = 0; i < kBlk; ++i) {
+        const float e0s = __fsub_rn(v0 + float(i), g.c0);
+        const f32x2 e0 = dup2(e0s), q0e = dup2(__fmul_rn(g.q00, e0s)), qb = dup2(__fmul_rn(g.q02x2, e0s));
+        f32x2 P0, P1, P2;  // the plane's sums of a, a e1, a e2
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            // row_a, row_b
+            const f32x2 A = fma2(fma2(q01, e1[p], q0e), e0, qe[p]);
+            const f32x2 B = fma2(q12, e1[p], qb);
+            f32x2 R0, R1;
+#pragma unroll
+            for (int k = 0; k < kBlk; ++k) {
+                const float4 gv = *reinterpret_cast<const float4*>(gs + grad_at(i, 2 * p, k));
+                const f32x2 gr = make_float2(gv.x, gv.y), gi = make_float2(gv.z, gv.w);
+                const f32x2 m = fma2(fma2(q22, e2[k], B), e2[k], A);  // row_m
+                const f32x2 x = mul2(m, scale);
+                const float wl = ex2_approx(x.x), wh = ex2_approx(x.y);
+                const f32x2 w = make_float2(m.x <= kCut ? wl : 0.f, m.y <= kCut ? wh : 0.f);
+                const f32x2 a = mul2(w, fma2(hi, gi, mul2(hr, gr)));
+                Dr = fma2(w, gr, Dr);
+                Di = fma2(w, gi, Di);
+                R0 = k ? add2(R0, a) : a;
+                R1 = k ? fma2(a, e2[k], R1) : mul2(a, e2[k]);
+                M22 = fma2(a, e2s[k], M22);
+            }
+            P0 = p ? add2(P0, R0) : R0;
+            P1 = p ? fma2(e1[p], R0, P1) : mul2(e1[p], R0);
+            P2 = p ? add2(P2, R1) : R1;
+            M11 = fma2(e1s[p], R0, M11);
+            M12 = fma2(e1[p], R1, M12);
+        }
+        const float p0 = sum2(P0), p1 = sum2(P1), p2 = sum2(P2), u = e0s * p0;
+        S0 += u;
+        S1 += p1;
+        S2 += p2;
+        M00 = fmaf(e0s, u, M00);
+        M01 = fmaf(e0s, p1, M01);
+        M02 = fmaf(e0s, p2, M02);
+    }
+    mom[0] = sum2(Dr); mom[1] = sum2(Di); mom[2] = S0; mom[3] = S1; mom[4] = S2;
+    mom[5] = M00; mom[6] = M01; mom[7] = M02; mom[8] = sum2(M11); mom[9] = sum2(M12);
+    mom[10] = sum2(M22); mom[11] = 0.f;
+}
+
+// block_moments for infinite, NaN or huge inputs: a voxel outside the cutoff takes part in no product, and
+// a Gaussian with no voxel inside adds exactly zero.
+__device__ __noinline__ void block_moments_guarded(const Rec& g, const float* gs, float v0, float v1, float v2,
+                                                   float mom[kMomStride]) {
+    const float hr = -0.5f * g.rho_r, hi = -0.5f * g.rho_i;
+    for (int i = 0; i < kMomStride; ++i) mom[i] = 0.f;
+    for (int i = 0; i < kBlk; ++i)
+        for (int j = 0; j < kBlk; ++j) {
+            const float e0 = __fsub_rn(v0 + float(i), g.c0), e1 = __fsub_rn(v1 + float(j), g.c1);
+            const float A = row_a(g, e0, e1), B = row_b(g, e0, e1);
+            for (int k = 0; k < kBlk; ++k) {
+                const float e2 = __fsub_rn(v2 + float(k), g.c2);
+                const float m = row_m(g.q22, A, B, e2);
+                if (!(m <= kCut)) continue;
+                const float gr = gs[grad_at(i, j, k)], gi = gs[grad_at(i, j, k) + 2];
+                const float w = ex2_approx(m * kNegHalfLog2e);
+                const float a = w * fmaf(hi, gi, hr * gr);
+                mom[0] = fmaf(w, gr, mom[0]);
+                mom[1] = fmaf(w, gi, mom[1]);
+                mom[2] = fmaf(a, e0, mom[2]);
+                mom[3] = fmaf(a, e1, mom[3]);
+                mom[4] = fmaf(a, e2, mom[4]);
+                mom[5] = fmaf(a * e0, e0, mom[5]);
+                mom[6] = fmaf(a * e0, e1, mom[6]);
+                mom[7] = fmaf(a * e0, e2, mom[7]);
+                mom[8] = fmaf(a * e1, e1, mom[8]);
+                mom[9] = fmaf(a * e1, e2, mom[9]);
+                mom[10] = fmaf(a * e2, e2, mom[10]);
+            }
+        }
+}
+
+// Whether a Gaussian needs block_moments_guarded.
 __device__ __forceinline__ bool needs_guard(const Rec& r) {
     return !(fabsf(r.rho_r) <= kBig && fabsf(r.rho_i) <= kBig && fabsf(r.c0) <= kBig && fabsf(r.c1) <= kBig &&
              fabsf(r.c2) <= kBig);
@@ -654,8 +681,8 @@ __device__ __forceinline__ void compat_emit_lane(const RenderArgs& a, const Rec&
 // up to kBwdCap kept Gaussians of its share of the tile's list, lists their (Gaussian, block) tasks
 // block by block, and deals the tasks to its lanes 32 at a time; a Gaussian's tasks add up in shared
 // memory in block order, so its pair total does not depend on which lanes ran them.
-constexpr int kBwdCap = 64;
-constexpr int kGradStride = kBlkVox + 2;  // float2 per block of the staged gradient: two blocks' rows in other banks
+constexpr int kBwdCap = 80;
+constexpr int kGradStride = 2 * kBlkVox + 4;  // floats per block of the staged gradient: two blocks' rows in other banks
 
 struct __align__(16) BwdStage {
     float4 rec[kBwdCap][3];
@@ -669,10 +696,12 @@ struct __align__(16) BwdStage {
 // Backward of one tile (RPL = 2) or of its half `sub` (RPL = 1).  One CTA barrier.
 template <bool COMPAT, bool DET, int RPL>
 __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile, int sub, BwdStage* stage,
-                                              float2* grad, int part) {
+                                              float* grad, int part) {
     static_assert(!DET || RPL == 2, "deterministic partials need the whole tile in one CTA");
     const int2 rg = a.ranges[tile];
-    if (rg.x >= rg.y) return;  // CTA-uniform
+    // a long list is shared by up to a.split CTAs
+    const int parts = min(a.split, (rg.y - rg.x + a.part - 1) / a.part);
+    if (part >= parts) return;  // CTA-uniform; also every CTA of an empty tile
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int d0, h0, w0;
     decode_tile(a, tile, d0, h0, w0);
@@ -686,7 +715,7 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
         const bool row_ok = gd < a.d && gh < a.h;
         const int64_t flat = (int64_t(gd) * a.h + gh) * a.w + gw;
         const int blk = (ld >> 2) * 4 + (lh >> 2) * 2 + bw;
-        float2* dst = grad + blk * kGradStride + ((ld & 3) * kBlk + (lh & 3)) * kBlk;
+        float* dst = grad + blk * kGradStride;
 #pragma unroll
         for (int k = 0; k < kBlk; ++k) {
             float2 x = make_float2(0.f, 0.f);
@@ -694,27 +723,33 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
                 x = COMPAT ? make_float2(__ldg(a.gv_r + flat + k), __ldg(a.gv_i + flat + k))
                            : __ldg(reinterpret_cast<const float2*>(a.gvol) + flat + k);
             guard |= !(fabsf(x.x) <= kBig && fabsf(x.y) <= kBig);
-            dst[k] = x;
+            dst[grad_at(ld & 3, lh & 3, k)] = x.x;
+            dst[grad_at(ld & 3, lh & 3, k) + 2] = x.y;
         }
     }
     guard = __syncthreads_or(guard);
 
     float ih[3];
     compat_ih<COMPAT>(a, ih);
+    constexpr int kWords = (kBwdCap + 31) / 32;
     BwdStage& S = stage[warp];
-    // list positions of this warp: first, first + stride, ... (part `part` of a.split CTAs)
-    const int stride = kWarps * a.split, first = part * kWarps + warp;
+    // list positions of this warp: first, first + stride, ... (part `part` of the tile's CTAs)
+    const int stride = kWarps * parts, first = part * kWarps + warp;
     const int mine = rg.y - rg.x > first ? (rg.y - rg.x - first + stride - 1) / stride : 0;
     const unsigned blocks = RPL == 2 ? 0xffu : 0xfu << (4 * sub);
+    const int32_t* ids = a.pair_ids + rg.x + first;
+    const bool mine_lane = lane < a.chunk;
+    // the next round's Gaussian, loaded one round ahead
+    int next = mine_lane && lane < mine ? __ldg(ids + stride * lane) : 0;
     for (int i0 = 0; i0 < mine;) {
         int kept = 0;
         for (; i0 < mine && kept + a.chunk <= kBwdCap; i0 += a.chunk) {
             Rec r;
-            int gid = 0;
+            const int gid = next;
             unsigned in = 0;
-            const bool listed = lane < min(a.chunk, mine - i0);
+            const bool listed = mine_lane && i0 + lane < mine;
+            if (mine_lane && i0 + a.chunk + lane < mine) next = __ldg(ids + stride * (i0 + a.chunk + lane));
             if (listed) {
-                gid = __ldg(a.pair_ids + rg.x + first + stride * (i0 + lane));
                 r = load_rec<COMPAT>(a, gid, ih);
                 in = blocks;
                 if (a.cull) {
@@ -744,13 +779,14 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
         __syncwarp();
         // tasks, block by block, each block's Gaussians in list order
         int tasks = 0;
-        unsigned m0 = lane < kept ? S.mask[lane] : 0u, m1 = lane + 32 < kept ? S.mask[lane + 32] : 0u;
-        static_assert(kBwdCap == 64, "two mask words per lane");
+        unsigned mask[kWords];
+#pragma unroll
+        for (int s = 0; s < kWords; ++s) mask[s] = lane + 32 * s < kept ? S.mask[lane + 32 * s] : 0u;
 #pragma unroll
         for (int b = 0; b < 8; ++b) {
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const bool hit = ((s ? m1 : m0) >> b) & 1u;
+            for (int s = 0; s < kWords; ++s) {
+                const bool hit = (mask[s] >> b) & 1u;
                 const unsigned bal = __ballot_sync(kFull, hit);
                 if (hit) S.task[tasks + __popc(bal & ((1u << lane) - 1u))] = uint16_t((lane + 32 * s) | (b << 8));
                 tasks += __popc(bal);
@@ -762,12 +798,18 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
             const unsigned task = S.task[on ? t0 + lane : tasks - 1];
             const int slot = task & 0xff, b = task >> 8;
             const Rec g = rec_of(S.rec[slot][0], S.rec[slot][1], S.rec[slot][2]);
-            const float2* gs = grad + b * kGradStride;
+            const float* gs = grad + b * kGradStride;
             const float v0 = float(d0 + (b >> 2) * kBlk), v1 = float(h0 + ((b >> 1) & 1) * kBlk),
                         v2 = float(w0 + (b & 1) * kBlk);
             float m[kMomStride];
-            if (guard || __any_sync(kFull, needs_guard(g))) block_moments<true>(g, gs, v0, v1, v2, m);
-            else block_moments<false>(g, gs, v0, v1, v2, m);
+            if (guard || __any_sync(kFull, needs_guard(g))) {
+                float mg[kMomStride];
+                block_moments_guarded(g, gs, v0, v1, v2, mg);
+#pragma unroll
+                for (int i = 0; i < kMomStride; ++i) m[i] = mg[i];
+            } else {
+                block_moments(g, gs, v0, v1, v2, m);
+            }
             // a Gaussian may have two of its blocks among these lanes: one block at a time
             const int b_end = __shfl_sync(kFull, b, 31);
             for (int bb = __shfl_sync(kFull, b, 0); bb <= b_end; ++bb) {
@@ -810,9 +852,9 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
 }
 
 template <bool COMPAT, bool DET, int RPL>
-__global__ void __launch_bounds__(kThreads, 5) k_backward8(const RenderArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) k_backward8(const RenderArgs a) {
     __shared__ __align__(16) BwdStage stage[kWarps];
-    __shared__ __align__(16) float2 grad[8 * kGradStride];
+    __shared__ __align__(16) float grad[8 * kGradStride];
     constexpr int subs = 2 / RPL;
     const int part = blockIdx.x % a.split, rest = blockIdx.x / a.split;
     backward_tile<COMPAT, DET, RPL>(a, rest / subs, rest % subs, stage, grad, part);
@@ -1335,9 +1377,9 @@ __global__ void __launch_bounds__(kThreads) k_forward8_batched(const BatchTable 
 }
 
 template <bool DET>
-__global__ void __launch_bounds__(kThreads, 5) k_backward8_batched(const BatchTable t) {
+__global__ void __launch_bounds__(kThreads, 4) k_backward8_batched(const BatchTable t) {
     __shared__ __align__(16) BwdStage stage[kWarps];
-    __shared__ __align__(16) float2 grad[8 * kGradStride];
+    __shared__ __align__(16) float grad[8 * kGradStride];
     __shared__ long long s_next;
     const int64_t total = t.tile_prefix[t.count];
     for (;;) {
@@ -1462,7 +1504,14 @@ void fill_shape(RenderArgs& a, gsv_shape s) {
     a.ntiles = int64_t((s.d + s.tile_size - 1) / s.tile_size) * a.nth * a.ntw;
     a.chunk = 32;
     a.cull = 1;
-    a.split = 1;
+    // Backward, 8^3 tiles: 592 CTAs are resident, so with few tiles a long list is worth two CTAs, with
+    // many it only adds half-filled groups.  Measured with 1 and 2 CTAs, a second one from 512 list
+    // positions on, us: 128x128x96/50k, 3072 tiles 208 and 192; 128x128x96/500k 468 and 429; 165^3/155k,
+    // 9261 tiles 526 and 537; 256x256x160/2M, 20480 tiles 2253 and 2330.  Below two resident rounds
+    // shorter lists are worth it too (from 256 on: 64^3/20k, 512 tiles 43 and 40; 100x84x60/20k, 1144
+    // tiles 113 and 88).
+    a.split = a.ntiles < 8 * 592 ? 2 : 1;
+    a.part = a.ntiles < 2 * 592 ? 256 : 512;
     const float sh[3] = {float(s.d), float(s.h), float(s.w)};
     for (int k = 0; k < 3; ++k) {
         a.hs[k] = sh[k] * 0.5f;
@@ -1561,7 +1610,7 @@ int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* 
     if (tuning) {
         a.chunk = tuning->chunk;
         a.cull = !(tuning->flags & GSV_TUNE_NO_CULL);
-        a.split = tuning->split > 1 ? tuning->split : 1;
+        if (tuning->split > 0) a.split = tuning->split;
     }
     if (ntiles * 2 * a.split > int64_t(INT32_MAX)) return GSV_ERR_INVALID_ARGUMENT;
     const int rpl = (tuning && !det) ? tuning->rows_per_lane : 2;  // deterministic: whole tiles
@@ -1679,7 +1728,7 @@ int gsv_tile_backward(const float* centers, const float* cov_inv, const float* d
     a.g_cov = grad_cov_inv;
     a.g_dr = grad_den_r;
     a.g_di = grad_den_i;
-    if (tile_size == 8) k_backward8<true, false, 2><<<unsigned(num_tiles), kThreads, 0, st>>>(a);
+    if (tile_size == 8) k_backward8<true, false, 2><<<unsigned(num_tiles * a.split), kThreads, 0, st>>>(a);
     else if (tile_size == 4)
         k_backward4<true, false><<<unsigned((num_tiles + kWarps - 1) / kWarps), kThreads, 0, st>>>(a);
     else k_backward_generic<true, false><<<unsigned(num_tiles), kThreads, 0, st>>>(a);
@@ -1729,6 +1778,7 @@ int gsv_batch_setup(const gsv_batch_item* items, int count, int flags, void* ws_
         a.offsets = cat<int64_t>(it.ws_gauss, G.offsets);
         a.capacity = it.capacity;
         a.chunk = (it.chunk >= 1 && it.chunk <= 32) ? it.chunk : 32;
+        a.split = 1;  // one work item per tile
         host[i] = a;
         tp[i + 1] = tp[i] + ntiles;
         gp[i + 1] = gp[i] + it.params.n;
