@@ -3,13 +3,12 @@
 Two knobs change speed but not results (every candidate evaluates the same
 (voxel, Gaussian) pairs of the same tile lists with the same arithmetic):
 
-* execution tile shape -- a CTA covers the whole 8^3 binning tile (two
-  8-voxel rows per lane) or a 4x8x8 half tile (one row per lane: fewer
-  registers, twice the CTAs);
-* Gaussian batch -- how many Gaussians a warp stages in shared memory at a
-  time (8, 16 or 32);
-* backward list split -- how many CTAs share one tile's Gaussian list in the
-  backward (1, 2 or 4): more CTAs for volumes with too few tiles to fill
+* execution tile shape -- a CTA covers the whole 8^3 binning tile or a 4x8x8
+  half tile (twice the CTAs, each staging the tile's list for itself);
+* Gaussian batch -- how many list positions a warp of the backward stages in
+  shared memory at a time (8, 16 or 32);
+* backward list split -- how many CTAs may share one tile's Gaussian list in
+  the backward (1, 2 or 4): more CTAs for volumes with too few tiles to fill
   the GPU.
 
 ``Autotuner.pick`` times every candidate's forward + backward on the binned
@@ -124,8 +123,7 @@ class Autotuner:
     def pick_tile_size(self, params, volume_shape, flags: int = 0) -> Tuple[int, GsvTuning, Dict[str, float]]:
         """Binning tile edge for a problem: times one whole step (preprocess,
         binning, forward, backward) at each edge of TILE_SIZES -- edge 8 with
-        its best execution shape (pick), edge 4 on the generic one-voxel-per-
-        thread kernels -- and keeps the fastest, cached like pick.  On a
+        its best execution shape (pick), edge 4 on its own kernels -- and keeps the fastest, cached like pick.  On a
         cubic volume the edges include the same (voxel, Gaussian) pairs and
         differ only by FP32 summation order.  On a non-cubic one the
         reference's radius 3 max_j(s_j hs_j) can cut a rotated anisotropic

@@ -129,9 +129,9 @@ def prepare_and_bin(params: Tuple[torch.Tensor, ...], shape: GsvShape, flags: in
 
 def work_census(plan: BinPlan, cull: bool = True) -> dict:
     """What the tile-8 render kernels do on a binned problem
-    (gsv_count_work): included candidates, candidates evaluated after the
-    extent cull, lanes issued by the exp / FMA blocks and kept slots without
-    an included voxel.  Synchronises the current stream."""
+    (gsv_count_work): included candidates, candidates evaluated (voxels of the
+    4x4x4 blocks the cull keeps), exponentials issued for them, and kept blocks
+    without an included voxel.  Synchronises the current stream."""
     out = torch.zeros(4, dtype=torch.int64, device=plan.device)
     tune = _lib.GsvTuning(2, 32, 0 if cull else _lib.GSV_TUNE_NO_CULL)
     check(lib.gsv_count_work(plan.shape, plan.n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.capacity or 0,

@@ -202,13 +202,13 @@ GSV_API int gsv_backward_batched(void* ws_batch, int count, int flags, void* str
 
 /* ---- execution tuning (results do not depend on it) ------------------ */
 
-/* No counterpart in the reference.  rows_per_lane: 2 = one CTA per 8^3 tile
- * (two 8-voxel rows per lane), 1 = one CTA per 4x8x8 half tile (one row per
- * lane; the deterministic backward always uses whole tiles).  chunk: number
- * of list positions a warp stages in shared memory at a time (1..32).  flags:
- * GSV_TUNE_NO_CULL turns off the extent cull (a Gaussian, or a 4x8x8 row
- * slot of it, whose conservative tight extent misses the CTA's voxels is
- * skipped; it contributes nothing there either way).  split: the
+/* No counterpart in the reference.  rows_per_lane: 2 = one CTA per 8^3 tile,
+ * 1 = one CTA per 4x8x8 half tile (the deterministic backward always uses
+ * whole tiles).  chunk: number of list positions a warp of the backward
+ * stages in shared memory at a time (1..32).  flags: GSV_TUNE_NO_CULL turns
+ * off the cull (a Gaussian is evaluated on the 4x4x4 blocks that its
+ * conservative tight extent and separating planes leave; it contributes
+ * nothing on the others either way).  split: the
  * backward lets up to `split` CTAs share a (half) tile's list when it is
  * long -- more CTAs for volumes whose tiles are too few to fill the GPU
  * (the forward ignores it).  Tile edge 8 only;
@@ -235,10 +235,9 @@ GSV_API int gsv_backward_ex(const gsv_params* params, gsv_shape shape, void* ws_
  * unchanged).  out: FOUR device uint64 counters, overwritten --
  *   [0] included candidates (Mahalanobis <= 9, voxel inside the volume),
  *   [1] candidates the kernels evaluate the quadratic for (voxels of the
- *       4x8x8 row slots the extent cull keeps),
- *   [2] lanes issued by the per-column exp / FMA blocks (32 per voxel column
- *       of a kept slot in which some lane is inside the cutoff),
- *   [3] kept slots without any included voxel.
+ *       4x4x4 blocks the cull keeps),
+ *   [2] exponentials they issue (every voxel of a kept block),
+ *   [3] kept blocks without any included voxel.
  * tuning (may be NULL): only GSV_TUNE_NO_CULL is read.  Tile edge 8 only.
  * Asynchronous on `stream`. */
 GSV_API int gsv_count_work(gsv_shape shape, int64_t n, const void* ws_gauss, const void* ws_pairs,
