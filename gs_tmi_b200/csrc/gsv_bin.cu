@@ -67,17 +67,19 @@ __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPre
 // kCsSeg; rows padded to whole words); k_colscan writes, per row and tile,
 // the position of the row's first pair of that tile in the sorted output
 // ("cs_pos": the column's exclusive prefix plus the tile's start, from a
-// single-pass scan of the tile totals) and the tile ranges; k_scatter walks
-// each row's Gaussians in id order and places their pairs.  The result
-// equals the stable radix sort's, which larger problems keep.  The counts
-// stay intact and k_scatter clears k_colscan's scan state, so binning may
+// single-pass scan of the tile totals) and the tile ranges; k_scatter places
+// each row's pairs.  The result equals the stable radix sort's, which larger
+// problems keep.  The counts stay intact and k_scatter clears k_colscan's scan state, so binning may
 // be repeated after one preprocess (e.g. with a larger capacity).
 constexpr int kCsSeg = 64;                                  // Gaussians per row: two warps of k_prepare
 constexpr int kCsRowsPerBlock = kPrepThreads / kCsSeg;      // rows per k_prepare block
-// k_scatter keeps kCsRowsPerBlock x ntiles int32 in shared memory: at most 48 KB, the size a
-// launch may use without a function attribute (none is set, also not inside a graph capture)
+// k_scatter keeps 12 bytes per tile in shared memory: at most 48 KB, the size a launch may use
+// without a function attribute (none is set, also not inside a graph capture)
 constexpr int64_t kCsMaxTiles = 3072;
-constexpr int64_t kCsMaxCells = int64_t(1) << 22;           // rows x tiles: 4 MB of counts, 16 MB of positions
+// rows x tiles: 16 MB of counts, 64 MB of positions.  128x128x96 (3072 tiles), preprocess and binning, radix
+// and counting sort: 100k Gaussians (4.8 M cells) 106 and 73 us, 200k 139 and 108, 300k (14 M) 160 and
+// 143, 500k (24 M) 200 and 258.
+constexpr int64_t kCsMaxCells = int64_t(1) << 24;
 constexpr int kCsCols = 32, kCsRowGroups = 32;              // k_colscan block: 32 columns x 32 row groups
 __host__ __device__ inline int64_t cs_rows(int64_t n) { return prep_blocks(n) * kCsRowsPerBlock; }
 __host__ __device__ inline int64_t cs_col_blocks(int64_t ntiles) { return (ntiles + kCsCols - 1) / kCsCols; }
@@ -587,23 +589,28 @@ __global__ void __launch_bounds__(kCsCols * kCsRowGroups) k_colscan(const uint8_
     }
 }
 
-// Placement pass of the counting sort: one warp per row of kCsSeg
-// Gaussians, kCsRowsPerBlock rows per block.  The warp copies its row of
-// positions to shared memory, then walks the row's Gaussians in ascending
-// id: the lanes take the Gaussian's tiles (distinct tiles, so no two lanes
-// share a counter), write its id at each tile's current position and advance
-// it.  Positions at or past `cap` are dropped (the overflow flag says so).
-// Block 0 also latches the capacity flags and clears k_colscan's ticket
-// counter and look-back words (k_colscan has finished: stream order).
-__global__ void __launch_bounds__(32 * kCsRowsPerBlock) k_scatter(const int32_t* __restrict__ pos_in,
-                                                                  const int4* __restrict__ boxes,
-                                                                  const int64_t* __restrict__ offsets, int64_t n,
-                                                                  int32_t ntiles, int64_t rows, DevShape s,
-                                                                  int64_t cap, int32_t* __restrict__ pair_ids,
-                                                                  Status* status, unsigned long long* lb,
-                                                                  int64_t lb_words) {
-    constexpr unsigned kAll = 0xffffffffu;
-    extern __shared__ int32_t cs_at[];  // [kCsRowsPerBlock][ntiles]
+// Placement pass of the counting sort: one block per row of kCsSeg Gaussians.
+// A pair's place is its row's position for that tile plus the number of the
+// row's earlier Gaussians in it.  Every tile has a word with a bit per Gaussian
+// of the row: all pairs set their bits (in any order), then read the bits below
+// their own, so no pair waits for another (a warp that walked the row's
+// Gaussians in order instead took 19 us for eight rows and 27 us for 783; this
+// takes 7 and 20 us).  A warp takes every kCsWarps-th Gaussian, its lanes
+// that Gaussian's tiles.  Positions at or past `cap` are dropped (the overflow
+// flag says so).  Block 0 also latches the capacity flags and clears
+// k_colscan's ticket counter and look-back words (k_colscan has finished:
+// stream order).
+constexpr int kCsWarps = 8;
+
+__global__ void __launch_bounds__(32 * kCsWarps) k_scatter(const int32_t* __restrict__ pos_in,
+                                                           const int4* __restrict__ boxes,
+                                                           const int64_t* __restrict__ offsets, int64_t n,
+                                                           int32_t ntiles, DevShape s, int64_t cap,
+                                                           int32_t* __restrict__ pair_ids, Status* status,
+                                                           unsigned long long* lb, int64_t lb_words) {
+    static_assert(kCsSeg == 64, "a tile's word has 64 bits");
+    extern __shared__ uint2 cs_bits[];  // [ntiles], then the row's positions
+    int32_t* at_t = reinterpret_cast<int32_t*>(cs_bits + ntiles);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) {
@@ -614,30 +621,51 @@ __global__ void __launch_bounds__(32 * kCsRowsPerBlock) k_scatter(const int32_t*
         }
         for (int64_t i = threadIdx.x; i < lb_words; i += blockDim.x) lb[i] = 0ull;
     }
-    const int64_t row = int64_t(blockIdx.x) * kCsRowsPerBlock + warp;
-    if (row >= rows) return;  // warp-uniform; no block barrier follows
-    int32_t* at_t = cs_at + warp * ntiles;
-    for (int t = lane; t < ntiles; t += 32) at_t[t] = pos_in[row * ntiles + t];
-    __syncwarp();
-    const int64_t g0 = row * kCsSeg;
-    for (int h = 0; h < kCsSeg; h += 32) {
-        const int64_t gl = g0 + h + lane;
-        const int4 mb = gl < n ? boxes[gl] : make_int4(0, 0, 0, 0);
-        for (int k = 0; k < 32; ++k) {  // the Gaussians in ascending id
-            const int cnt = __shfl_sync(kAll, mb.w, k);
-            const int bx = __shfl_sync(kAll, mb.x, k), by = __shfl_sync(kAll, mb.y, k),
-                      bz = __shfl_sync(kAll, mb.z, k);
-            if (cnt <= 0) continue;  // warp-uniform
-            const int32_t gid = int32_t(g0 + h + k);
+    const int64_t row = blockIdx.x, g0 = row * kCsSeg;
+    if (g0 >= n) return;  // block-uniform
+    // lane j of warp w holds the box of the warp's j-th Gaussian
+    constexpr int kMine = kCsSeg / kCsWarps;
+    const int64_t gl = g0 + warp + kCsWarps * lane;
+    const int4 mb = lane < kMine && gl < n ? boxes[gl] : make_int4(0, 0, 0, 0);
+    for (int t0 = threadIdx.x; t0 < ntiles; t0 += 4 * blockDim.x) {  // four loads in flight
+        int32_t v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = t0 + i * blockDim.x;
+            v[i] = t < ntiles ? __ldg(pos_in + row * ntiles + t) : 0;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = t0 + i * blockDim.x;
+            if (t < ntiles) {
+                cs_bits[t] = make_uint2(0u, 0u);
+                at_t[t] = v[i];
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int k = 0; k < kMine; ++k) {
+            const int cnt = __shfl_sync(0xffffffffu, mb.w, k);
+            const int bx = __shfl_sync(0xffffffffu, mb.x, k), by = __shfl_sync(0xffffffffu, mb.y, k),
+                      bz = __shfl_sync(0xffffffffu, mb.z, k);
+            const int j = warp + kCsWarps * k;  // place in the row
+            const uint32_t bit = 1u << (j & 31);
             const float r1 = box_rcp(bz), r2 = box_rcp(bz >> 16);
             for (int c = lane; c < cnt; c += 32) {
                 const int32_t t = box_tile_small(s, bx, by, bz, r1, r2, c);
-                const int32_t p = at_t[t];
-                if (p < cap) pair_ids[p] = gid;
-                at_t[t] = int32_t(min(int64_t(p) + 1, cap));
+                if (pass == 0) {
+                    atomicOr(j < 32 ? &cs_bits[t].x : &cs_bits[t].y, bit);
+                } else {
+                    const uint2 w = cs_bits[t];
+                    const int before = j < 32 ? __popc(w.x & (bit - 1u)) : __popc(w.x) + __popc(w.y & (bit - 1u));
+                    const int64_t p = int64_t(at_t[t]) + before;
+                    if (p < cap) pair_ids[p] = int32_t(g0 + j);
+                }
             }
-            __syncwarp();
         }
+        if (pass == 0) __syncthreads();
     }
 }
 
@@ -657,12 +685,12 @@ int sync_total(const GaussLayout& L, void* ws, int64_t n, int64_t* total_host, c
     return GSV_OK;
 }
 
-// Dynamic shared memory of k_prepare's byte counters and of k_scatter's positions.  Neither
+// Dynamic shared memory of k_prepare's byte counters and of k_scatter's words and positions.  Neither
 // kernel declares static shared memory beyond a few words, and both stay within the 48 KB a
 // launch may use without a function attribute.
 int cs_prep_smem_bytes(int64_t ntiles) { return int(kCsRowsPerBlock * ((ntiles + 3) / 4) * int64_t(sizeof(uint32_t))); }
-int cs_scatter_smem_bytes(int64_t ntiles) { return int(kCsRowsPerBlock * ntiles * int64_t(sizeof(int32_t))); }
-static_assert(kCsRowsPerBlock * kCsMaxTiles * 4 <= 48 * 1024, "k_scatter's positions exceed 48 KB");
+int cs_scatter_smem_bytes(int64_t ntiles) { return int(ntiles * int64_t(sizeof(uint2) + sizeof(int32_t))); }
+static_assert(kCsMaxTiles * (sizeof(uint2) + sizeof(int32_t)) <= 48 * 1024, "k_scatter's words and positions exceed 48 KB");
 static_assert(kCsRowsPerBlock * kCsMaxTiles <= 40 * 1024, "k_prepare's counters leave no room for its static words");
 
 // Shared tail of both binning flavours.  Counting sort (k_colscan,
@@ -697,8 +725,8 @@ int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, s
             at<uint8_t>(ws_gauss, G.cs_mat), at<int32_t>(ws_gauss, G.cs_pos), rows, T, cap, ranges, status, lb_cs);
         GSV_LAUNCH_CHECK();
         const int smem = cs_scatter_smem_bytes(T);
-        k_scatter<<<unsigned(prep_blocks(n)), 32 * kCsRowsPerBlock, smem, st>>>(
-            at<int32_t>(ws_gauss, G.cs_pos), at<int4>(ws_gauss, G.box), offsets, n, T, rows, s, cap, vals_out, status,
+        k_scatter<<<unsigned(rows), 32 * kCsWarps, smem, st>>>(
+            at<int32_t>(ws_gauss, G.cs_pos), at<int4>(ws_gauss, G.box), offsets, n, T, s, cap, vals_out, status,
             lb_cs, cs_col_blocks(T));
         GSV_LAUNCH_CHECK();
         return GSV_OK;

@@ -325,7 +325,7 @@ __device__ __forceinline__ void block_moments(const Rec& g, const float* gs, flo
                 const f32x2 x = mul2(m, scale);
                 const float wl = ex2_approx(x.x), wh = ex2_approx(x.y);
                 const f32x2 w = make_float2(m.x <= kCut ? wl : 0.f, m.y <= kCut ? wh : 0.f);
-                const f32x2 a = mul2(w, fma2(hi, gi, mul2(hr, gr)));
+                const f32x2 a = mul2(w, fma2(hr, gr, mul2(hi, gi)));
                 Dr = fma2(w, gr, Dr);
                 Di = fma2(w, gi, Di);
                 R0 = k ? add2(R0, a) : a;
@@ -511,26 +511,26 @@ __device__ __noinline__ void add_gaussians_guarded(BlockSums& s, const float4* r
     add_gaussians<true>(s, recs, list, n, lane);
 }
 
-// Sums the warp's four partial blocks ((0 + 2) + (1 + 3)) and stores the block: lane group q keeps
-// columns 2 (q / 2), + 1 of row q % 2 of the lane's two.
+// Sums the warp's four partial blocks ((0 + 1) + (2 + 3)) and stores the block: lane group q keeps
+// columns 2 (q % 2), + 1 of row q / 2 of the lane's two.
 template <bool PLANAR>
 __device__ __forceinline__ void store_block(const RenderArgs& a, const BlockSums& s, int d0, int h0, int w0, int lane) {
-    const bool kp = lane & 16, row = lane & 8;
+    const bool kp = lane & 8, row = lane & 16;
     f32x2 re[2], im[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const f32x2 sr = kp ? s.re[i] : s.re[i + 2], kr = kp ? s.re[i + 2] : s.re[i];
         const f32x2 si = kp ? s.im[i] : s.im[i + 2], ki = kp ? s.im[i + 2] : s.im[i];
-        re[i].x = kr.x + __shfl_xor_sync(kFull, sr.x, 16);
-        re[i].y = kr.y + __shfl_xor_sync(kFull, sr.y, 16);
-        im[i].x = ki.x + __shfl_xor_sync(kFull, si.x, 16);
-        im[i].y = ki.y + __shfl_xor_sync(kFull, si.y, 16);
+        re[i].x = kr.x + __shfl_xor_sync(kFull, sr.x, 8);
+        re[i].y = kr.y + __shfl_xor_sync(kFull, sr.y, 8);
+        im[i].x = ki.x + __shfl_xor_sync(kFull, si.x, 8);
+        im[i].y = ki.y + __shfl_xor_sync(kFull, si.y, 8);
     }
     float vr[2], vi[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        vr[i] = (row ? re[i].y : re[i].x) + __shfl_xor_sync(kFull, row ? re[i].x : re[i].y, 8);
-        vi[i] = (row ? im[i].y : im[i].x) + __shfl_xor_sync(kFull, row ? im[i].x : im[i].y, 8);
+        vr[i] = (row ? re[i].y : re[i].x) + __shfl_xor_sync(kFull, row ? re[i].x : re[i].y, 16);
+        vi[i] = (row ? im[i].y : im[i].x) + __shfl_xor_sync(kFull, row ? im[i].x : im[i].y, 16);
     }
     const int gd = d0 + ((lane >> 1) & 3), gh = h0 + 2 * (lane & 1) + (row ? 1 : 0), gw = w0 + (kp ? 2 : 0);
     if (gd >= a.d || gh >= a.h) return;
