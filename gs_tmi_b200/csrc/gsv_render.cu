@@ -54,7 +54,8 @@ struct RenderArgs {
     const float* gv_r;  // planar
     const float* gv_i;
     float* accum;     // [n, 12] moments (native, atomics)
-    float* partials;  // [pairs, 12] moments (native, deterministic), at each pair's emission index
+    float* partials;  // [pairs, 12] moments (native, deterministic), at each pair's emission index ...
+    uint8_t* kept;    // ... of the pairs marked here; the others add nothing
     const int64_t* offsets;  // per-Gaussian first emission index (binning scan)
     int64_t capacity;        // pair capacity (bound of every emission index)
     float* g_center;  // compat outputs
@@ -192,12 +193,14 @@ __device__ __forceinline__ void compat_emit(const RenderArgs& a, const Rec& g, i
 // Emission index of the pair (Gaussian gid, tile (td, th, tw)): the
 // Gaussian's first index plus the tile's raster position in its tile box --
 // where binning emitted it.  Per-pair partials stored at this index lie
-// contiguously per Gaussian, in tile raster order.
-__device__ __forceinline__ int64_t emission_index(const RenderArgs& a, int gid, int td, int th, int tw) {
+// contiguously per Gaussian, in tile raster order.  -1: past the pair capacity
+// (overflow, flagged), the partial is dropped.
+__device__ __forceinline__ int32_t emission_index(const RenderArgs& a, int gid, int td, int th, int tw) {
     const int4 b = __ldg(a.boxes + gid);
     const int t0 = b.x & 0xffff, t1 = (b.x >> 16) & 0xffff, t2 = b.y & 0xffff;
     const int n1 = b.z & 0xffff, n2 = (b.z >> 16) & 0xffff;
-    return __ldg(a.offsets + gid) + (int64_t(td - t0) * n1 + (th - t1)) * n2 + (tw - t2);
+    const int64_t e = __ldg(a.offsets + gid) + (int64_t(td - t0) * n1 + (th - t1)) * n2 + (tw - t2);
+    return e < a.capacity ? int32_t(e) : -1;
 }
 
 // ---------------------------------------------------------------------------
@@ -727,11 +730,6 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
                 }
             }
             const unsigned keep = __ballot_sync(kFull, in != 0);
-            if (DET && listed && !in) {  // dropped pair: its partial is zero
-                float4* dst = reinterpret_cast<float4*>(a.partials +
-                                                        emission_index(a, gid, d0 >> 3, h0 >> 3, w0 >> 3) * kMomStride);
-                dst[0] = dst[1] = dst[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
             if (in) {
                 const int pos = kept + __popc(keep & ((1u << lane) - 1u));
 #pragma unroll
@@ -741,7 +739,7 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
                 }
                 S.gid[pos] = gid;
                 S.mask[pos] = uint8_t(in);
-                if (DET) S.pidx[pos] = int32_t(emission_index(a, gid, d0 >> 3, h0 >> 3, w0 >> 3));
+                if (DET) S.pidx[pos] = emission_index(a, gid, d0 >> 3, h0 >> 3, w0 >> 3);
             }
             kept += __popc(keep);
         }
@@ -807,6 +805,7 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
                 }
                 compat_emit_lane(a, rec_of(S.rec[k][0], S.rec[k][1], S.rec[k][2]), gid, m, ih);
             } else {
+                if (DET && S.pidx[k] < 0) continue;
                 float4* dst = reinterpret_cast<float4*>(DET ? a.partials + int64_t(S.pidx[k]) * kMomStride
                                                             : a.accum + int64_t(gid) * kMomStride);
 #pragma unroll
@@ -814,6 +813,7 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
                     if (DET) dst[i] = S.mom[k][i];
                     else atomicAdd(dst + i, S.mom[k][i]);
                 }
+                if (DET) a.kept[S.pidx[k]] = 1;
             }
         }
         __syncwarp();
@@ -981,22 +981,16 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward4(const RenderArgs a) {
             const bool listed = base + lane < rg.y;
             Rec r;
             bool hit = false;
-            int64_t e = 0;
             if (listed) {
                 hit = load_hit4<COMPAT>(a, gid, d0, h0, w0, ih, r) || !a.cull;
-                if (DET) e = emission_index(a, gid, d0 >> 2, h0 >> 2, w0 >> 2);
             }
             const unsigned kept = __ballot_sync(kFull, hit);
-            if (DET && listed && !hit) {  // dropped pair: its partial is zero
-                float4* dst = reinterpret_cast<float4*>(a.partials + e * kMomStride);
-                dst[0] = dst[1] = dst[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
             if (hit) {
                 const int at = (tail + __popc(kept & ((1u << lane) - 1u))) & (kBwd4Ring - 1);
 #pragma unroll
                 for (int i = 0; i < 3; ++i) S.rec[at][i] = rec_quad(r, i);
                 S.gid[at] = gid;
-                if (DET) S.pidx[at] = int32_t(e);
+                if (DET) S.pidx[at] = emission_index(a, gid, d0 >> 2, h0 >> 2, w0 >> 2);
             }
             tail += __popc(kept);
         }
@@ -1015,7 +1009,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward4(const RenderArgs a) {
         } else {
             block_moments(g, S.grad, v0, v1, v2, m);
         }
-        if (on) {
+        if (on && !(DET && S.pidx[at] < 0)) {
             if (COMPAT) {
                 compat_emit_lane(a, g, gid, m, ih);
             } else {
@@ -1027,6 +1021,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward4(const RenderArgs a) {
                     if (DET) dst[i] = x;
                     else atomicAdd(dst + i, x);
                 }
+                if (DET) a.kept[S.pidx[at]] = 1;
             }
         }
         head = min(head + 32, tail);
@@ -1088,7 +1083,7 @@ template <bool COMPAT, bool DET>
 __global__ void __launch_bounds__(kThreads) k_backward_generic(const RenderArgs a) {
     __shared__ Rec srec[32];
     __shared__ int sgid[32];
-    __shared__ int64_t sidx[32];
+    __shared__ int32_t sidx[32];
     __shared__ float sred[kWarps][kMom];
     const int64_t tile = blockIdx.x;
     const int2 rg = a.ranges[tile];
@@ -1160,7 +1155,8 @@ __global__ void __launch_bounds__(kThreads) k_backward_generic(const RenderArgs 
                 if (COMPAT) {
                     compat_emit(a, g, gid, spread, lane, ih);
                 } else if (DET) {
-                    if (lane < kMom) a.partials[sidx[j] * kMomStride + lane] = t;
+                    if (lane < kMom && sidx[j] >= 0) a.partials[int64_t(sidx[j]) * kMomStride + lane] = t;
+                    if (lane == 0 && sidx[j] >= 0) a.kept[sidx[j]] = 1;
                 } else {
                     if (lane < kMom) atomicAdd(a.accum + int64_t(gid) * kMomStride + lane, t);
                 }
@@ -1176,52 +1172,120 @@ __global__ void __launch_bounds__(kThreads) k_backward_generic(const RenderArgs 
 // tail of the reference), in FP32.
 // ---------------------------------------------------------------------------
 
-// Deterministic moments of Gaussian g, one warp: the Gaussian's per-pair
-// partials sit contiguously at its emission indices, in tile raster order;
-// lane l sums entries l, l + 32, ... and a fixed xor tree sums the lanes.
-// The order depends only on the tile box, so the result is bitwise
-// reproducible.  Writes the moments where the atomic backward accumulates
-// them.
-__device__ __forceinline__ void gather_det_warp(const RenderArgs& a, int64_t g, int lane) {
-    float mo[kMom];
+// What the deterministic gather reads of one volume.
+struct DetView {
+    const int4* boxes;
+    const int64_t* offsets;
+    const float* partials;
+    const uint8_t* kept;
+    int64_t capacity;
+};
+__device__ __forceinline__ DetView det_view(const RenderArgs& a) {
+    return DetView{a.boxes, a.offsets, a.partials, a.kept, a.capacity};
+}
+
+// Deterministic moments of 4 R Gaussians (base .. base + 4 R - 1 of `total`), R rounds
+// of four with eight lanes each: a Gaussian's per-pair partials sit contiguously at
+// its emission indices, in tile raster order, and the pairs the backward kept are
+// marked.  Lane l of the eight takes entries l, l + 8, ... and a fixed xor tree sums
+// the lanes (a Gaussian of more than kGatherGroup pairs: the whole warp, l + 32, ...).
+// Either order depends only on the tile box, so the result is bitwise reproducible
+// and does not depend on R.  Lane 4 r + q ends with the moments of round r's
+// Gaussian q.  `locate(x, view, g)`: volume and row of Gaussian x.
+constexpr int kGatherGroup = 256;
+
+__device__ __forceinline__ void add_partial(float mo[kMom], const float* src) {
+    const float4* p = reinterpret_cast<const float4*>(src);
+    const float4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
+    mo[0] += x.x; mo[1] += x.y; mo[2] += x.z; mo[3] += x.w;
+    mo[4] += y.x; mo[5] += y.y; mo[6] += y.z; mo[7] += y.w;
+    mo[8] += z.x; mo[9] += z.y; mo[10] += z.z;
+}
+
+// First emission index of a Gaussian's pairs and how many of them have partials.
+__device__ __forceinline__ int det_pairs(const DetView& v, int64_t g, int64_t& first) {
+    first = v.offsets[g];
+    const int64_t left = v.capacity - first;  // past the capacity (overflow, flagged) there are none
+    return int(left <= 0 ? 0 : min(int64_t(v.boxes[g].w), left));
+}
+
+template <int R, typename Locate>
+__device__ __forceinline__ void gather_det(const Locate& locate, int64_t base, int64_t total, int lane, float mo[kMom]) {
 #pragma unroll
     for (int i = 0; i < kMom; ++i) mo[i] = 0.f;
-    const int cnt = a.boxes[g].w;
-    const int64_t first = a.offsets[g];
-    for (int c = lane; c < cnt; c += 32) {
-        const int64_t e = first + c;
-        if (e >= a.capacity) break;  // pair capacity overflow (flagged): no such partial
-        const float4* src = reinterpret_cast<const float4*>(a.partials + e * kMomStride);
-        const float4 x = src[0], y = src[1], z = src[2];
-        mo[0] += x.x; mo[1] += x.y; mo[2] += x.z; mo[3] += x.w;
-        mo[4] += y.x; mo[5] += y.y; mo[6] += y.z; mo[7] += y.w;
-        mo[8] += z.x; mo[9] += z.y; mo[10] += z.z;
+    // lane 4 r + q: where its Gaussian's marks and partials are
+    unsigned long long my_kept = 0, my_partials = 0;
+    int my_cnt = 0;
+    if (lane < 4 * R && base + lane < total) {
+        DetView v;
+        int64_t g, first;
+        locate(base + lane, v, g);
+        my_cnt = det_pairs(v, g, first);
+        my_kept = (unsigned long long)(v.kept + first);
+        my_partials = (unsigned long long)(v.partials + first * kMomStride);
     }
+#pragma unroll 1
+    for (int r = 0; r < R; ++r) {
+        const int from = 4 * r + (lane >> 3);
+        const uint8_t* kept = reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, my_kept, from));
+        const float* partials = reinterpret_cast<const float*>(__shfl_sync(kFull, my_partials, from));
+        const int cnt = __shfl_sync(kFull, my_cnt, from);
+        float part[kMom];
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1)
+        for (int i = 0; i < kMom; ++i) part[i] = 0.f;
+        if (cnt <= kGatherGroup) {
+            for (int c = lane & 7; c < cnt; c += 16) {  // two entries in flight
+                const bool on0 = __ldg(kept + c), on1 = c + 8 < cnt && __ldg(kept + c + 8);
+                if (on0) add_partial(part, partials + c * kMomStride);
+                if (on1) add_partial(part, partials + (c + 8) * kMomStride);
+            }
+        }
 #pragma unroll
-        for (int i = 0; i < kMom; ++i) mo[i] += __shfl_xor_sync(0xffffffffu, mo[i], off);
-    if (lane == 0) {
-        float4* dst = reinterpret_cast<float4*>(a.accum + g * kMomStride);
-        dst[0] = make_float4(mo[0], mo[1], mo[2], mo[3]);
-        dst[1] = make_float4(mo[4], mo[5], mo[6], mo[7]);
-        dst[2] = make_float4(mo[8], mo[9], mo[10], 0.f);
+        for (int off = 4; off >= 1; off >>= 1)
+#pragma unroll
+            for (int i = 0; i < kMom; ++i) part[i] += __shfl_xor_sync(kFull, part[i], off);
+        for (unsigned big = __ballot_sync(kFull, cnt > kGatherGroup && (lane & 7) == 0); big; big &= big - 1) {
+            const int src = __ffs(big) - 1;
+            const uint8_t* bk = reinterpret_cast<const uint8_t*>(__shfl_sync(kFull, (unsigned long long)kept, src));
+            const float* bp = reinterpret_cast<const float*>(__shfl_sync(kFull, (unsigned long long)partials, src));
+            const int n = __shfl_sync(kFull, cnt, src);
+            float all[kMom];
+#pragma unroll
+            for (int i = 0; i < kMom; ++i) all[i] = 0.f;
+            for (int c = lane; c < n; c += 32)
+                if (__ldg(bk + c)) add_partial(all, bp + int64_t(c) * kMomStride);
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+                for (int i = 0; i < kMom; ++i) all[i] += __shfl_xor_sync(kFull, all[i], off);
+            if ((lane & ~7) == src)
+#pragma unroll
+                for (int i = 0; i < kMom; ++i) part[i] = all[i];
+        }
+#pragma unroll
+        for (int i = 0; i < kMom; ++i) {
+            const float t = __shfl_sync(kFull, part[i], (lane & 3) * 8);
+            if ((lane >> 2) == r) mo[i] = t;
+        }
     }
 }
 
-// Chain rule of one Gaussian from its 11 moments (accum).  The moments are
-// cleared once read: the preprocess clears them too, so the atomic backward
-// always starts from zero without a memset of its own.
-__device__ __forceinline__ void finalize_one(const RenderArgs& a, int64_t g) {
+// Moments of one Gaussian from the atomic accumulators, which are cleared once
+// read: the preprocess clears them too, so the atomic backward always starts
+// from zero without a memset of its own.
+__device__ __forceinline__ void take_moments(const RenderArgs& a, int64_t g, float mo[kMom]) {
+    float4* acc4 = reinterpret_cast<float4*>(a.accum + g * kMomStride);
+    const float4 x = acc4[0], y = acc4[1], z = acc4[2];
+    acc4[0] = acc4[1] = acc4[2] = make_float4(0.f, 0.f, 0.f, 0.f);
+    mo[0] = x.x; mo[1] = x.y; mo[2] = x.z; mo[3] = x.w;
+    mo[4] = y.x; mo[5] = y.y; mo[6] = y.z; mo[7] = y.w;
+    mo[8] = z.x; mo[9] = z.y; mo[10] = z.z;
+}
+
+// Chain rule of one Gaussian from its 11 moments.
+__device__ __forceinline__ void finalize_one(const RenderArgs& a, int64_t g, const float mo[kMom]) {
     const gsv_params& p = a.prm;
     const gsv_grads& out = a.grd;
-    float mo[kMom];
-#pragma unroll
-    for (int i = 0; i < kMom; ++i) mo[i] = a.accum[g * kMomStride + i];
-    {
-        float4* acc4 = reinterpret_cast<float4*>(a.accum + g * kMomStride);
-        acc4[0] = acc4[1] = acc4[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
     const Rec R = a.recs[g];
     // dL/dcenter_vox, then dcenter/dpositions = 0.5 * shape = hs   (:284).
     // The reference sums this over included pairs only: a Gaussian with none
@@ -1297,14 +1361,20 @@ __device__ __forceinline__ void finalize_one(const RenderArgs& a, int64_t g) {
 __global__ void __launch_bounds__(256) k_finalize(const RenderArgs a) {
     const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (g >= a.prm.n) return;
-    finalize_one(a, g);
+    float mo[kMom];
+    take_moments(a, g, mo);
+    finalize_one(a, g, mo);
 }
 
-// One warp per Gaussian (deterministic backward).
-__global__ void __launch_bounds__(256) k_gather_det(const RenderArgs a) {
-    const int64_t g = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (g >= a.prm.n) return;  // warp-uniform
-    gather_det_warp(a, g, threadIdx.x & 31);
+// The deterministic backward's gather and chain rule, 4 R Gaussians per warp.
+template <int R>
+__global__ void __launch_bounds__(256) k_finalize_det(const RenderArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int64_t base = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * (4 * R);
+    const DetView view = det_view(a);
+    float mo[kMom];
+    gather_det<R>([&](int64_t x, DetView& v, int64_t& g) { v = view; g = x; }, base, a.prm.n, lane, mo);
+    if (lane < 4 * R && base + lane < a.prm.n) finalize_one(a, base + lane, mo);
 }
 
 // ---------------------------------------------------------------------------
@@ -1318,7 +1388,7 @@ struct BatchTable {
     RenderArgs* items;
     int64_t* tile_prefix;   // [count + 1]
     int64_t* gauss_prefix;  // [count + 1]
-    int64_t* cap_prefix;    // [count + 1]
+    int64_t* cap_prefix;    // [count + 1]  deterministic: 16-byte words of marks
     unsigned long long* counters;  // [2]: forward, backward work counters
     int count;
     int det;
@@ -1371,17 +1441,41 @@ __global__ void __launch_bounds__(256) k_finalize_batched(const BatchTable t) {
     for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total;
          x += int64_t(gridDim.x) * blockDim.x) {
         const int i = find_item(t.gauss_prefix, t.count, x);
-        finalize_one(t.items[i], x - t.gauss_prefix[i]);
+        float mo[kMom];
+        take_moments(t.items[i], x - t.gauss_prefix[i], mo);
+        finalize_one(t.items[i], x - t.gauss_prefix[i], mo);
     }
 }
 
-// One warp per Gaussian of every volume (deterministic backward).
-__global__ void __launch_bounds__(256) k_gather_det_batched(const BatchTable t) {
+// k_finalize_det over every volume's Gaussians.
+__global__ void __launch_bounds__(256) k_finalize_det_batched(const BatchTable t) {
+    constexpr int R = 4;
+    const int lane = threadIdx.x & 31;
     const int64_t total = t.gauss_prefix[t.count];
     const int64_t warps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t x = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; x < total; x += warps) {
-        const int i = find_item(t.gauss_prefix, t.count, x);  // warp-uniform
-        gather_det_warp(t.items[i], x - t.gauss_prefix[i], threadIdx.x & 31);
+    for (int64_t base = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * (4 * R); base < total;
+         base += warps * (4 * R)) {  // warp-uniform
+        float mo[kMom];
+        gather_det<R>(
+            [&](int64_t x, DetView& v, int64_t& g) {
+                const int i = find_item(t.gauss_prefix, t.count, x);
+                v = det_view(t.items[i]);
+                g = x - t.gauss_prefix[i];
+            },
+            base, total, lane, mo);
+        if (lane < 4 * R && base + lane < total) {
+            const int i = find_item(t.gauss_prefix, t.count, base + lane);
+            finalize_one(t.items[i], base + lane - t.gauss_prefix[i], mo);
+        }
+    }
+}
+
+// Clears every volume's marks of kept pairs (16 at a time; the marks' buffer is longer than its capacity).
+__global__ void __launch_bounds__(256) k_clear_kept_batched(const BatchTable t) {
+    const int64_t total = t.cap_prefix[t.count];
+    for (int64_t x = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total; x += int64_t(gridDim.x) * blockDim.x) {
+        const int i = find_item(t.cap_prefix, t.count, x);
+        reinterpret_cast<uint4*>(t.items[i].kept)[x - t.cap_prefix[i]] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -1562,12 +1656,13 @@ int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* 
     a.gvol = grad_volume;
     a.accum = mat<float>(ws_gauss, G.accum);
     a.partials = det ? mat<float>(ws_pairs, P.partials) : nullptr;
+    a.kept = det ? mat<uint8_t>(ws_pairs, P.keys_in) : nullptr;  // the unsorted keys are no longer needed
     a.offsets = cat<int64_t>(ws_gauss, G.offsets);
     a.boxes = cat<int4>(ws_gauss, G.box);
     a.capacity = capacity;
     // The atomic accumulators are zero here: the preprocess clears them and
     // k_finalize clears them again after reading.  The deterministic mode
-    // writes every listed pair's partial and its gather overwrites them.
+    // marks the pairs whose partials it writes and does not touch them.
     if (tuning) {
         a.chunk = tuning->chunk;
         a.cull = !(tuning->flags & GSV_TUNE_NO_CULL);
@@ -1577,6 +1672,7 @@ int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* 
     const int rpl = (tuning && !det) ? tuning->rows_per_lane : 2;  // deterministic: whole tiles
     const unsigned sp = unsigned(a.split);
     if (capacity > 0) {
+        if (det) GSV_CUDA_TRY(cudaMemsetAsync(a.kept, 0, size_t(capacity), st));
         if (shape.tile_size == 8) {
             if (det) k_backward8<false, true, 2><<<unsigned(ntiles) * sp, kThreads, 0, st>>>(a);
             else if (rpl == 2) k_backward8<false, false, 2><<<unsigned(ntiles) * sp, kThreads, 0, st>>>(a);
@@ -1592,11 +1688,10 @@ int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* 
     }
     a.prm = *p;
     a.grd = *grads;
-    if (det) {
-        k_gather_det<<<grid_for(n * 32, 256), 256, 0, st>>>(a);
-        GSV_LAUNCH_CHECK();
-    }
-    k_finalize<<<grid_for(n, 256), 256, 0, st>>>(a);
+    // four Gaussians a warp while the warps are few, 32 (every lane busy in the chain rule) above
+    if (det && capacity > 0 && n < 131072) k_finalize_det<1><<<grid_for(n, 32), 256, 0, st>>>(a);
+    else if (det && capacity > 0) k_finalize_det<8><<<grid_for(n, 256), 256, 0, st>>>(a);
+    else k_finalize<<<grid_for(n, 256), 256, 0, st>>>(a);
     GSV_LAUNCH_CHECK();
     return GSV_OK;
 }
@@ -1733,6 +1828,7 @@ int gsv_batch_setup(const gsv_batch_item* items, int count, int flags, void* ws_
         a.gvol = it.grad_volume;
         a.accum = mat<float>(const_cast<void*>(it.ws_gauss), G.accum);
         a.partials = det && it.capacity > 0 ? mat<float>(const_cast<void*>(it.ws_pairs), P.partials) : nullptr;
+        a.kept = det && it.capacity > 0 ? mat<uint8_t>(const_cast<void*>(it.ws_pairs), P.keys_in) : nullptr;
         a.prm = it.params;
         a.grd = it.grads;
         a.boxes = cat<int4>(it.ws_gauss, G.box);
@@ -1743,7 +1839,7 @@ int gsv_batch_setup(const gsv_batch_item* items, int count, int flags, void* ws_
         host[i] = a;
         tp[i + 1] = tp[i] + ntiles;
         gp[i + 1] = gp[i] + it.params.n;
-        cp[i + 1] = cp[i] + (det ? it.capacity : 0);
+        cp[i + 1] = cp[i] + (det ? (it.capacity + 15) / 16 : 0);
     }
     if (rc == GSV_OK) {
         cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1811,15 +1907,17 @@ int gsv_backward_batched(void* ws_batch, int count, int flags, void* stream) {
     // every volume's accumulators are zero: its preprocess cleared them and
     // k_finalize(_batched) clears them again after reading
     const int grid = persistent_grid(reinterpret_cast<const void*>(k_finalize_batched), 256);
-    if (det) k_backward8_batched<true><<<persistent_grid(reinterpret_cast<const void*>(k_backward8_batched<true>), kThreads), kThreads, 0, st>>>(t);
-    else k_backward8_batched<false><<<persistent_grid(reinterpret_cast<const void*>(k_backward8_batched<false>), kThreads), kThreads, 0, st>>>(t);
-    GSV_LAUNCH_CHECK();
     if (det) {
-        k_gather_det_batched<<<persistent_grid(reinterpret_cast<const void*>(k_gather_det_batched), 256), 256, 0,
-                               st>>>(t);
+        k_clear_kept_batched<<<grid, 256, 0, st>>>(t);
         GSV_LAUNCH_CHECK();
+        k_backward8_batched<true><<<persistent_grid(reinterpret_cast<const void*>(k_backward8_batched<true>), kThreads), kThreads, 0, st>>>(t);
+        GSV_LAUNCH_CHECK();
+        k_finalize_det_batched<<<grid, 256, 0, st>>>(t);
+    } else {
+        k_backward8_batched<false><<<persistent_grid(reinterpret_cast<const void*>(k_backward8_batched<false>), kThreads), kThreads, 0, st>>>(t);
+        GSV_LAUNCH_CHECK();
+        k_finalize_batched<<<grid, 256, 0, st>>>(t);
     }
-    k_finalize_batched<<<grid, 256, 0, st>>>(t);
     GSV_LAUNCH_CHECK();
     return GSV_OK;
 }

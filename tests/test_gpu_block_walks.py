@@ -93,3 +93,33 @@ def test_counting_sort_at_its_largest_row_count(cuda_device):
 
     gs = synthetic.random_gaussians(300_000, (128, 128, 96), seed=2)
     _same_lists(_prepare(_params(gs, cuda_device), _shape((128, 128, 96), 8)))
+
+
+@pytest.mark.parametrize("ts", [8, 4, 5])
+def test_deterministic_backward_over_capacity_stays_in_its_buffers(ts, cuda_device):
+    """A static deterministic plan whose capacity is half the pairs: the overflow is flagged, and the
+    marks and partials of pairs past the capacity are dropped (guard bytes behind the pair workspace
+    stay as they were)."""
+    import ctypes
+
+    from gs_tmi_b200 import _lib
+    from gs_tmi_b200._lib import GsvGrads, GsvParams, check, lib
+    from gs_tmi_b200.tile_voxelizer import StaticPlan, TileVoxelizer, _ptr, _shape, _stream
+
+    shape = (40, 40, 40)
+    gs = synthetic.random_gaussians(3000, shape, seed=3)
+    ps = [t.to(cuda_device) for t in gs.tensors()]
+    total = TileVoxelizer(shape, ts).count_pairs(ps[0], ps[1])
+    plan = StaticPlan(_shape(shape, ts), 3000, cuda_device, total // 2, flags=_lib.GSV_BACKWARD_DETERMINISTIC)
+    guarded = torch.full((plan.pair_bytes + (1 << 22),), 77, dtype=torch.uint8, device=cuda_device)
+    plan.ws_pairs = guarded
+    gv = synthetic.upstream_grad(shape, seed=4).to(cuda_device)
+    outs = [torch.empty_like(t) for t in ps]
+    gp, gg, st = GsvParams(*(t.data_ptr() for t in ps), 3000), GsvGrads(*(o.data_ptr() for o in outs)), _stream(cuda_device)
+    check(lib.gsv_prepare(ctypes.byref(gp), plan.shape, _ptr(plan.ws_gauss), plan.gauss_bytes, None, st), "prepare")
+    check(lib.gsv_bin(plan.shape, 3000, _ptr(plan.ws_gauss), _ptr(guarded), plan.pair_bytes, plan.capacity, st), "bin")
+    check(lib.gsv_backward(ctypes.byref(gp), plan.shape, _ptr(plan.ws_gauss), _ptr(guarded), plan.capacity, _ptr(gv),
+                           ctypes.byref(gg), plan.flags, st), "backward")
+    assert plan.read_status(st)[1] & _lib.GSV_FLAG_CAPACITY_OVERFLOW
+    assert all(torch.isfinite(o).all() for o in outs)
+    assert (guarded[plan.pair_bytes:] == 77).all()
