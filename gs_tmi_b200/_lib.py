@@ -90,6 +90,7 @@ SIGNATURES = {
     "gsv_pair_workspace_bytes": (_sz, [_i64, _S, ctypes.c_int]),
     "gsv_prepare": (ctypes.c_int, [_P, _S, _vp, _sz, _i64p, _vp]),
     "gsv_prepare_live": (ctypes.c_int, [_P, _vp, _S, _vp, _sz, _i64p, _vp]),
+    "gsv_prepare_strided": (ctypes.c_int, [_P, _i64, _vp, _S, _vp, _sz, _i64p, _i32p, _vp]),
     "gsv_bin": (ctypes.c_int, [_S, _i64, _vp, _vp, _sz, _i64, _vp]),
     "gsv_bin_ex": (ctypes.c_int, [_S, _i64, _vp, _vp, _sz, _i64, ctypes.c_int, _vp]),
     "gsv_bin_views": (ctypes.c_int, [_S, _i64, _vp, _vp, _i64, ctypes.POINTER(_vp), ctypes.POINTER(_vp)]),
@@ -98,6 +99,8 @@ SIGNATURES = {
     "gsv_forward": (ctypes.c_int, [_S, _i64, _vp, _vp, _i64, _vp, _vp]),
     "gsv_forward_ex": (ctypes.c_int, [_S, _i64, _vp, _vp, _i64, _vp, ctypes.c_void_p, _vp]),
     "gsv_backward_ex": (ctypes.c_int, [_P, _S, _vp, _vp, _i64, _vp, _G, ctypes.c_int, ctypes.c_void_p, _vp]),
+    "gsv_backward_strided": (ctypes.c_int, [_P, _S, _vp, _vp, _i64, _vp, _G, _i64, ctypes.c_int, ctypes.c_void_p,
+                                            _vp]),
     "gsv_backward": (ctypes.c_int, [_P, _S, _vp, _vp, _i64, _vp, _G, ctypes.c_int, _vp]),
     "gsv_batch_workspace_bytes": (_sz, [ctypes.c_int]),
     "gsv_batch_setup": (ctypes.c_int, [ctypes.POINTER(GsvBatchItem), ctypes.c_int, ctypes.c_int, _vp, _sz, _vp]),

@@ -24,7 +24,7 @@ import torch
 
 from . import _lib
 from ._lib import GsvBatchItem, GsvGrads, GsvParams, check, lib
-from .tile_voxelizer import StaticPlan, _f32, _ptr, _shape, _stream, prepare_and_bin
+from .tile_voxelizer import StaticPlan, _f32, _Prepared, _ptr, _shape, _stream
 
 
 def _item(shape, params, plan, volume, grad_volume=None, grads=None, chunk=32) -> GsvBatchItem:
@@ -52,8 +52,9 @@ class _BatchFn(torch.autograd.Function):
         groups = [tuple(_f32(t) for t in flat[5 * i:5 * i + 5]) for i in range(len(bv.shapes))]
         plans, vols, items = [], [], []
         with torch.cuda.device(dev):
-            for shape, params in zip(bv.gshapes, groups):
-                plan = prepare_and_bin(params, shape, bv.flags)
+            prepared = [_Prepared(params, shape, bv.flags) for shape, params in zip(bv.gshapes, groups)]
+            for shape, params, prep in zip(bv.gshapes, groups, prepared):
+                plan = prep.bin()
                 vol = torch.empty((shape.d, shape.h, shape.w), dtype=torch.complex64, device=dev)
                 plans.append(plan)
                 vols.append(vol)

@@ -97,17 +97,11 @@ __host__ __device__ inline size_t status_bytes(int64_t n, int64_t ntiles) {
 
 GaussLayout gauss_layout(int64_t n, const ShapeInfo& si) {
     GaussLayout L{};
-    size_t scan_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const int64_t*)nullptr, (int64_t*)nullptr,
-                                  int(n + 1));
-    L.scan_tmp_bytes = scan_bytes;
     size_t o = 0;
     L.rec = o;      o = align_up(o + size_t(n) * sizeof(Rec));
     L.ext = o;      o = align_up(o + size_t(n) * sizeof(float4));
     L.box = o;      o = align_up(o + size_t(n) * sizeof(int4));
-    L.counts = o;   o = align_up(o + size_t(n + 1) * sizeof(int64_t));
     L.offsets = o;  o = align_up(o + size_t(n + 1) * sizeof(int64_t));
-    L.scan_tmp = o; o = align_up(o + scan_bytes);
     L.ranges = o;   o = align_up(o + size_t(si.ntiles) * sizeof(int2));
     L.accum = o;    o = align_up(o + size_t(n) * kMomStride * sizeof(float));
     L.status = o;   o = align_up(o + status_bytes(n, si.ntiles));
@@ -263,16 +257,8 @@ __device__ int64_t lookback(unsigned long long* lb, int64_t bid, int64_t block_t
     return base;
 }
 
-// Tile id of pair `c` (0-based, raster order) of a Gaussian's packed tile box.
-__device__ __forceinline__ int32_t box_tile(const DevShape& s, int bx, int by, int bz, int32_t c) {
-    const int32_t t0 = bx & 0xffff, t1 = (bx >> 16) & 0xffff, t2 = by & 0xffff;
-    const int32_t n1 = bz & 0xffff, n2 = (bz >> 16) & 0xffff;
-    const int32_t k = c % n2, r = c / n2;
-    const int32_t jj = r % n1, i = r / n1;
-    return ((t0 + i) * s.nt[1] + (t1 + jj)) * s.nt[2] + (t2 + k);
-}
-
-// box_tile for the counting sort, where the pair index and both box extents
+// Tile id of pair `c` (0-based, raster order) of a Gaussian's packed tile box,
+// for the counting sort, where the pair index and both box extents
 // are below 4096 (they are at most the tile count, <= kCsMaxTiles): the two
 // integer divisions become trunc((x + 0.5) * rcp(n)) in IEEE single
 // precision, exact for 0 <= x < 4096 and 1 <= n <= 4096 (every pair checked
@@ -291,15 +277,58 @@ __device__ __forceinline__ int32_t box_tile_small(const DevShape& s, int bx, int
 }
 __device__ __forceinline__ float box_rcp(int field) { return __frcp_rn(float(max(field & 0xffff, 1))); }
 
+// The exclusive scan of the Gaussians' pair counts into `offsets`
+// (offsets[n] = pair total, also in Status::total), inside the kernel that
+// counts them, a thread per Gaussian.  Blocks take their position in the scan
+// from a counter in the status region, so every block a block waits for has
+// already started.
+__device__ __forceinline__ int64_t scan_ticket(Status* status) {
+    __shared__ int bid_s;
+    if (threadIdx.x == 0) bid_s = atomicAdd(&status->pad[1], 1);
+    __syncthreads();
+    return bid_s;
+}
+
+struct PairScan {
+    int64_t first;     // this Gaussian's first pair, counted within the block
+    int64_t warp_end;  // one past the warp's last
+};
+
+__device__ __forceinline__ PairScan scan_counts(int64_t cnt, int64_t n, int64_t bid, int64_t* __restrict__ offsets,
+                                                Status* status) {
+    __shared__ int64_t warp_tot[kPrepThreads / 32];
+    __shared__ int64_t block_base;
+    const int64_t g = bid * kPrepThreads + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    __syncthreads();
+    int64_t warp_base = 0, block_tot = 0;
+#pragma unroll
+    for (int w = 0; w < kPrepThreads / 32; ++w) {
+        if (w < warp) warp_base += warp_tot[w];
+        block_tot += warp_tot[w];
+    }
+    if (warp == 0) {
+        const int64_t base = lookback(reinterpret_cast<unsigned long long*>(status + 1), bid, block_tot, status, lane);
+        if (lane == 0) block_base = base;
+    }
+    __syncthreads();
+    const int64_t first = warp_base + incl - cnt;
+    if (g <= n) offsets[g] = block_base + first;
+    if (g == n) status->total = block_base + first;
+    return PairScan{first, warp_base + warp_tot[warp]};
+}
+
 // Preprocess (center, radius, quadratic-form coefficients, tight extent, tile
 // box) of one Gaussian per thread, the clearing of its backward moment
 // accumulators, and the exclusive scan of the Gaussians'
-// pair counts into `offsets` (offsets[n] = pair total) in the same launch.
-// Blocks take their position in the scan from a counter in the status
-// region, so every block a block waits for has already started; it waits
-// only for its predecessors' published totals, each wait bounded (on
-// time-out GSV_FLAG_SCAN_STALLED is latched and the block publishes anyway,
-// so no later block waits the full limit again).  With `cs_mat` the block
+// pair counts into `offsets` in the same launch (scan_counts).  With `cs_mat` the block
 // also counts its pairs per tile for each of its kCsRowsPerBlock rows and
 // writes those rows of cs_mat.  A row's count in one tile is at most kCsSeg
 // (< 256), so the counters are bytes, four to a word, in shared memory
@@ -309,19 +338,14 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
                                                           const float* __restrict__ scl,
                                                           const float* __restrict__ rot,
                                                           const float* __restrict__ dr,
-                                                          const float* __restrict__ di, int64_t n,
+                                                          const float* __restrict__ di, int64_t dstride, int64_t n,
                                                           const int32_t* __restrict__ live, DevShape s,
                                                           Rec* __restrict__ recs, float4* __restrict__ ext,
                                                           int4* __restrict__ boxes,
                                                           int64_t* __restrict__ offsets, Status* status,
                                                           uint8_t* __restrict__ cs_mat, int32_t ntiles,
                                                           float* __restrict__ accum) {
-    __shared__ int bid_s;
-    __shared__ int64_t warp_tot[kPrepThreads / 32];
-    __shared__ int64_t block_base;
-    if (threadIdx.x == 0) bid_s = atomicAdd(&status->pad[1], 1);
-    __syncthreads();
-    const int64_t bid = bid_s;
+    const int64_t bid = scan_ticket(status);
     const int64_t g = bid * kPrepThreads + threadIdx.x;
     int64_t cnt = 0;
     int4 box = make_int4(0, 0, 0, 0);
@@ -355,7 +379,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
         Rec R;
         R.c0 = c[0]; R.c1 = c[1]; R.c2 = c[2];
         R.q00 = qc[0]; R.q01x2 = qc[1]; R.q02x2 = qc[2]; R.q11 = qc[3]; R.q12x2 = qc[4]; R.q22 = qc[5];
-        R.rho_r = dr[g]; R.rho_i = di[g]; R.pad = 0.0f;
+        R.rho_r = dr[g * dstride]; R.rho_i = di[g * dstride]; R.pad = 0.0f;
         recs[g] = R;
         float4 x = tight_extent(qc);
         x.w = plane_threshold(R);
@@ -368,28 +392,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
         }
         boxes[g] = box;
     }
-    // block-wide inclusive scan of the counts
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    int64_t warp_base = 0, block_tot = 0;
-#pragma unroll
-    for (int w = 0; w < kPrepThreads / 32; ++w) {
-        if (w < warp) warp_base += warp_tot[w];
-        block_tot += warp_tot[w];
-    }
-    if (warp == 0) {
-        const int64_t base = lookback(reinterpret_cast<unsigned long long*>(status + 1), bid, block_tot, status, lane);
-        if (lane == 0) block_base = base;
-    }
-    __syncthreads();
-    if (g <= n) offsets[g] = block_base + warp_base + incl - cnt;
+    const PairScan sc = scan_counts(cnt, n, bid, offsets, status);
     if (cs_mat == nullptr) return;  // block-uniform
 
     // Per-row tile counts.  The warp's pairs occupy the block-local range
@@ -403,9 +407,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
     __syncthreads();
     {
         constexpr unsigned kAll = 0xffffffffu;
-        const long long o = warp_base + incl - cnt;
+        const long long o = sc.first;
         const long long wstart = __shfl_sync(kAll, o, 0);
-        const long long wend = warp_base + warp_tot[warp];
+        const long long wend = sc.warp_end;
         uint32_t* row = cs_hist + (warp * 32 / kCsSeg) * words;
         const float rcp1 = box_rcp(box.z), rcp2 = box_rcp(box.z >> 16);
         for (long long base = wstart; base < wend; base += 32) {
@@ -432,23 +436,26 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
     for (int i = threadIdx.x; i < kCsRowsPerBlock * words; i += kPrepThreads) dst[i] = cs_hist[i];
 }
 
-__global__ void __launch_bounds__(256) k_count_compat(const float* __restrict__ center,
-                                                      const float* __restrict__ radius, int64_t n,
-                                                      DevShape s, int4* __restrict__ boxes,
-                                                      int64_t* __restrict__ counts, Status* status) {
-    const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g == 0) counts[n] = 0;
-    if (g >= n) return;
-    float c[3] = {center[g * 3], center[g * 3 + 1], center[g * 3 + 2]};
-    int4 box;
-    int64_t cnt = tile_box(s, c, radius[g], &box);
-    if (cnt <= 0) {
-        atomicOr(&status->flags, GSV_FLAG_EMPTY_BOX);
-        cnt = 0;
-        box.w = 0;
+// Tile boxes, pair counts and their scan for the reference-signature binning.
+__global__ void __launch_bounds__(kPrepThreads) k_count_compat(const float* __restrict__ center,
+                                                               const float* __restrict__ radius, int64_t n,
+                                                               DevShape s, int4* __restrict__ boxes,
+                                                               int64_t* __restrict__ offsets, Status* status) {
+    const int64_t bid = scan_ticket(status);
+    const int64_t g = bid * kPrepThreads + threadIdx.x;
+    int64_t cnt = 0;
+    if (g < n) {
+        float c[3] = {center[g * 3], center[g * 3 + 1], center[g * 3 + 2]};
+        int4 box;
+        cnt = tile_box(s, c, radius[g], &box);
+        if (cnt <= 0) {
+            atomicOr(&status->flags, GSV_FLAG_EMPTY_BOX);
+            cnt = 0;
+            box.w = 0;
+        }
+        boxes[g] = box;
     }
-    boxes[g] = box;
-    counts[g] = cnt;
+    scan_counts(cnt, n, bid, offsets, status);
 }
 
 // One thread per Gaussian writes its (tile, gid) pairs in raster order.
@@ -676,12 +683,13 @@ int grid_for(int64_t items, int block) {
     return int(g);
 }
 
-int sync_total(const GaussLayout& L, void* ws, int64_t n, int64_t* total_host, cudaStream_t st) {
-    int64_t total = 0;
-    GSV_CUDA_TRY(cudaMemcpyAsync(&total, at<int64_t>(ws, L.offsets) + n, sizeof(int64_t),
-                                 cudaMemcpyDeviceToHost, st));
+// Flags and pair total of the last count, in one copy; synchronises the stream.
+int read_status(const GaussLayout& L, const void* ws, int64_t* total, int32_t* flags, cudaStream_t st) {
+    Status s{};
+    GSV_CUDA_TRY(cudaMemcpyAsync(&s, at<Status>(ws, L.status), sizeof(Status), cudaMemcpyDeviceToHost, st));
     GSV_CUDA_TRY(cudaStreamSynchronize(st));
-    *total_host = total;
+    if (total) *total = s.total;
+    if (flags) *flags = s.flags;
     return GSV_OK;
 }
 
@@ -793,8 +801,9 @@ size_t gsv_pair_workspace_bytes(int64_t capacity, gsv_shape shape, int flags) {
     return pair_layout(capacity, si, flags).total;
 }
 
-static int prepare_impl(const gsv_params* p, const int32_t* live, gsv_shape shape, void* ws_gauss,
-                        size_t ws_gauss_bytes, int64_t* total_pairs_host, void* stream) {
+static int prepare_impl(const gsv_params* p, int64_t density_stride, const int32_t* live, gsv_shape shape,
+                        void* ws_gauss, size_t ws_gauss_bytes, int64_t* total_pairs_host, int32_t* flags_host,
+                        void* stream) {
     ShapeInfo si = shape_info(shape);
     if (!si.ok || !p || p->n < 0 || p->n >= int64_t(INT32_MAX) || !ws_gauss) return GSV_ERR_INVALID_ARGUMENT;
     const int64_t n = p->n;
@@ -808,24 +817,31 @@ static int prepare_impl(const gsv_params* p, const int32_t* live, gsv_shape shap
     GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
     const int smem = L.cs ? cs_prep_smem_bytes(si.ntiles) : 0;
     k_prepare<<<unsigned(prep_blocks(n)), kPrepThreads, smem, st>>>(
-        p->positions, p->scales, p->rotations, p->density_r, p->density_i, n, live, dev_shape(si),
+        p->positions, p->scales, p->rotations, p->density_r, p->density_i, density_stride, n, live, dev_shape(si),
         at<Rec>(ws_gauss, L.rec), at<float4>(ws_gauss, L.ext), at<int4>(ws_gauss, L.box),
         at<int64_t>(ws_gauss, L.offsets), status, L.cs ? at<uint8_t>(ws_gauss, L.cs_mat) : nullptr,
         int32_t(si.ntiles), at<float>(ws_gauss, L.accum));
     GSV_LAUNCH_CHECK();
-    if (total_pairs_host) return sync_total(L, ws_gauss, n, total_pairs_host, st);
+    if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, flags_host, st);
     return GSV_OK;
 }
 
 int gsv_prepare(const gsv_params* p, gsv_shape shape, void* ws_gauss, size_t ws_gauss_bytes,
                 int64_t* total_pairs_host, void* stream) {
-    return prepare_impl(p, nullptr, shape, ws_gauss, ws_gauss_bytes, total_pairs_host, stream);
+    return prepare_impl(p, 1, nullptr, shape, ws_gauss, ws_gauss_bytes, total_pairs_host, nullptr, stream);
 }
 
 int gsv_prepare_live(const gsv_params* p, const int32_t* live, gsv_shape shape, void* ws_gauss,
                      size_t ws_gauss_bytes, int64_t* total_pairs_host, void* stream) {
     if (!live) return GSV_ERR_INVALID_ARGUMENT;
-    return prepare_impl(p, live, shape, ws_gauss, ws_gauss_bytes, total_pairs_host, stream);
+    return prepare_impl(p, 1, live, shape, ws_gauss, ws_gauss_bytes, total_pairs_host, nullptr, stream);
+}
+
+int gsv_prepare_strided(const gsv_params* p, int64_t density_stride, const int32_t* live, gsv_shape shape,
+                        void* ws_gauss, size_t ws_gauss_bytes, int64_t* total_pairs_host, int32_t* flags_host,
+                        void* stream) {
+    if (density_stride < 1) return GSV_ERR_INVALID_ARGUMENT;
+    return prepare_impl(p, density_stride, live, shape, ws_gauss, ws_gauss_bytes, total_pairs_host, flags_host, stream);
 }
 
 int gsv_bin_ex(gsv_shape shape, int64_t n, void* ws_gauss, void* ws_pairs, size_t ws_pairs_bytes,
@@ -855,7 +871,7 @@ int gsv_status_views(gsv_shape shape, int64_t n, void* ws_gauss, int32_t** flags
     if (!si.ok || n < 0 || !ws_gauss) return GSV_ERR_INVALID_ARGUMENT;
     const GaussLayout L = gauss_layout(n, si);
     if (flags) *flags = &at<Status>(ws_gauss, L.status)->flags;
-    if (total_pairs) *total_pairs = at<int64_t>(ws_gauss, L.offsets) + n;
+    if (total_pairs) *total_pairs = &at<Status>(ws_gauss, L.status)->total;
     return GSV_OK;
 }
 
@@ -864,17 +880,7 @@ int gsv_read_status(gsv_shape shape, int64_t n, const void* ws_gauss, int64_t* t
     ShapeInfo si = shape_info(shape);
     if (!si.ok || n < 0 || !ws_gauss) return GSV_ERR_INVALID_ARGUMENT;
     const GaussLayout L = gauss_layout(n, si);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int64_t total = 0;
-    Status s{};
-    GSV_CUDA_TRY(cudaMemcpyAsync(&total, at<int64_t>(ws_gauss, L.offsets) + n, sizeof(int64_t),
-                                 cudaMemcpyDeviceToHost, st));
-    GSV_CUDA_TRY(cudaMemcpyAsync(&s, at<Status>(ws_gauss, L.status), sizeof(Status),
-                                 cudaMemcpyDeviceToHost, st));
-    GSV_CUDA_TRY(cudaStreamSynchronize(st));
-    if (total_pairs) *total_pairs = total;
-    if (flags) *flags = s.flags;
-    return GSV_OK;
+    return read_status(L, ws_gauss, total_pairs, flags, static_cast<cudaStream_t>(stream));
 }
 
 int gsv_build_tile_pairs_count(const float* center_vox, const float* radius_vox, int64_t n,
@@ -887,16 +893,12 @@ int gsv_build_tile_pairs_count(const float* center_vox, const float* radius_vox,
     if (ws_gauss_bytes < L.total) return GSV_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Status* status = at<Status>(ws_gauss, L.status);
-    GSV_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(Status), st));
-    k_count_compat<<<grid_for(n + 1, 256), 256, 0, st>>>(center_vox, radius_vox, n, dev_shape(si),
-                                                         at<int4>(ws_gauss, L.box),
-                                                         at<int64_t>(ws_gauss, L.counts), status);
+    GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
+    k_count_compat<<<unsigned(prep_blocks(n)), kPrepThreads, 0, st>>>(center_vox, radius_vox, n, dev_shape(si),
+                                                                      at<int4>(ws_gauss, L.box),
+                                                                      at<int64_t>(ws_gauss, L.offsets), status);
     GSV_LAUNCH_CHECK();
-    size_t scan_bytes = L.scan_tmp_bytes;
-    GSV_CUDA_TRY(cub::DeviceScan::ExclusiveSum(at<void>(ws_gauss, L.scan_tmp), scan_bytes,
-                                               at<int64_t>(ws_gauss, L.counts),
-                                               at<int64_t>(ws_gauss, L.offsets), int(n + 1), st));
-    if (total_pairs_host) return sync_total(L, ws_gauss, n, total_pairs_host, st);
+    if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, nullptr, st);
     return GSV_OK;
 }
 

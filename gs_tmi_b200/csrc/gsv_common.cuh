@@ -171,8 +171,7 @@ __device__ __forceinline__ float row_m(float q22, float a, float b, float e2) {
 __host__ __device__ inline size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct GaussLayout {
-    size_t rec, ext, box, counts, offsets, scan_tmp, ranges, accum, status, cs_mat, cs_pos, total;
-    size_t scan_tmp_bytes;
+    size_t rec, ext, box, offsets, ranges, accum, status, cs_mat, cs_pos, total;
     bool cs;  // the counting-sort binning applies (cs_mat: per-row tile counts, cs_pos: positions)
 };
 
@@ -181,11 +180,15 @@ struct PairLayout {
     size_t sort_tmp_bytes;
 };
 
-// Status word (first 64 bytes of the status region).
+// Status word (first 64 bytes of the status region).  total: the pair total, beside the flags so that
+// one copy reads both.
 struct Status {
     int32_t flags;
-    int32_t pad[15];
+    int32_t pad[3];
+    int64_t total;
+    int32_t rest[10];
 };
+static_assert(sizeof(Status) == 64, "Status must be 64 bytes");
 
 }  // namespace gsv
 

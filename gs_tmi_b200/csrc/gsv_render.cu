@@ -69,6 +69,7 @@ struct RenderArgs {
     // finalize
     gsv_params prm;
     gsv_grads grd;
+    int64_t dstride;  // element stride of the density gradients
     const int4* boxes;
 };
 
@@ -1297,8 +1298,8 @@ __device__ __forceinline__ void finalize_one(const RenderArgs& a, int64_t g, con
     out.positions[g * 3 + 0] = dc0 * a.hs[0];
     out.positions[g * 3 + 1] = dc1 * a.hs[1];
     out.positions[g * 3 + 2] = dc2 * a.hs[2];
-    out.density_r[g] = mo[0];
-    out.density_i[g] = mo[1];
+    out.density_r[g * a.dstride] = mo[0];
+    out.density_i[g * a.dstride] = mo[1];
     // dL/dM (normalised units), symmetric.
     float G[9];
     G[0] = mo[5] * a.ih[0] * a.ih[0];
@@ -1559,6 +1560,7 @@ void fill_shape(RenderArgs& a, gsv_shape s) {
     a.ntiles = int64_t((s.d + s.tile_size - 1) / s.tile_size) * a.nth * a.ntw;
     a.chunk = 32;
     a.cull = 1;
+    a.dstride = 1;
     // Backward, 8^3 tiles: 592 CTAs are resident, so with few tiles a long list is worth two CTAs, with
     // many it only adds half-filled groups.  Measured with 1 and 2 CTAs, a second one from 512 list
     // positions on, us: 128x128x96/50k, 3072 tiles 208 and 192; 128x128x96/500k 468 and 429; 165^3/155k,
@@ -1633,7 +1635,13 @@ int gsv_backward(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* ws_
 int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* ws_pairs, int64_t capacity,
                     const float* grad_volume, const gsv_grads* grads, int flags, const gsv_tuning* tuning,
                     void* stream) {
-    if (!tuning_ok(tuning)) return GSV_ERR_INVALID_ARGUMENT;
+    return gsv_backward_strided(p, shape, ws_gauss, ws_pairs, capacity, grad_volume, grads, 1, flags, tuning, stream);
+}
+
+int gsv_backward_strided(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* ws_pairs, int64_t capacity,
+                         const float* grad_volume, const gsv_grads* grads, int64_t density_stride, int flags,
+                         const gsv_tuning* tuning, void* stream) {
+    if (!tuning_ok(tuning) || density_stride < 1) return GSV_ERR_INVALID_ARGUMENT;
     GaussLayout G;
     PairLayout P;
     int64_t ntiles = 0;
@@ -1688,6 +1696,7 @@ int gsv_backward_ex(const gsv_params* p, gsv_shape shape, void* ws_gauss, void* 
     }
     a.prm = *p;
     a.grd = *grads;
+    a.dstride = density_stride;
     // four Gaussians a warp while the warps are few, 32 (every lane busy in the chain rule) above
     if (det && capacity > 0 && n < 131072) k_finalize_det<1><<<grid_for(n, 32), 256, 0, st>>>(a);
     else if (det && capacity > 0) k_finalize_det<8><<<grid_for(n, 256), 256, 0, st>>>(a);

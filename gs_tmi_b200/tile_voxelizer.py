@@ -107,24 +107,44 @@ def _raise_flags(flags: int, total: int):
         raise RuntimeError(f"{total} (tile, Gaussian) pairs exceed the int32 tile ranges")
 
 
+def _pointers(params) -> Tuple[Tuple[Optional[int], ...], int]:
+    """Addresses of (pos, scl, rot, density_r, density_i) and the densities' stride.  params: those
+    five, (pos, scl, rot, density) with an interleaved complex64 density, or without densities (the
+    backward reads none)."""
+    if len(params) == 4:
+        den = params[3].data_ptr()
+        return (*(t.data_ptr() for t in params[:3]), den or None, den + 4 if den else None), 2
+    return (*(t.data_ptr() for t in params), *(None,) * (5 - len(params))), 1
+
+
+class _Prepared:
+    """A preprocess on its way: the launch now, the pair total and the sort later, so that several
+    volumes' preprocesses run before the first total is waited for."""
+
+    def __init__(self, params, shape: GsvShape, flags: int = 0):
+        dev = params[0].device
+        self.stream = _stream(dev)
+        self.plan = plan = BinPlan(shape, int(params[0].shape[0]), dev, flags)
+        ptrs, stride = _pointers(params)
+        gp = GsvParams(*ptrs, plan.n)
+        check(lib.gsv_prepare_strided(ctypes.byref(gp), stride, None, shape, _ptr(plan.ws_gauss), plan.gauss_bytes,
+                                      None, None, self.stream), "gsv_prepare")
+
+    def bin(self) -> BinPlan:
+        plan = self.plan
+        total, fl = plan.read_status(self.stream)
+        _raise_flags(fl, total)
+        plan.total = total
+        plan.alloc_pairs(total)
+        check(lib.gsv_bin(plan.shape, plan.n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.pair_bytes,
+                          plan.capacity, self.stream), "gsv_bin")
+        return plan
+
+
 def prepare_and_bin(params: Tuple[torch.Tensor, ...], shape: GsvShape, flags: int = 0) -> BinPlan:
     """Preprocess + bin on the current stream; reads the pair total back
     (one host sync, as the reference does at tile_voxelizer.py:118)."""
-    pos, scl, rot, dr, di = params
-    dev = pos.device
-    n = int(pos.shape[0])
-    st = _stream(dev)
-    plan = BinPlan(shape, n, dev, flags)
-    gp = GsvParams(pos.data_ptr(), scl.data_ptr(), rot.data_ptr(), dr.data_ptr(), di.data_ptr(), n)
-    check(lib.gsv_prepare(ctypes.byref(gp), shape, _ptr(plan.ws_gauss), plan.gauss_bytes, None, st),
-          "gsv_prepare")
-    total, fl = plan.read_status(st)
-    _raise_flags(fl, total)
-    plan.total = total
-    plan.alloc_pairs(total)
-    check(lib.gsv_bin(shape, n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.pair_bytes, plan.capacity, st),
-          "gsv_bin")
-    return plan
+    return _Prepared(params, shape, flags).bin()
 
 
 def work_census(plan: BinPlan, cull: bool = True) -> dict:
@@ -140,8 +160,24 @@ def work_census(plan: BinPlan, cull: bool = True) -> dict:
     return {"included": inc, "evaluated": ev, "exp_block_lanes": lanes, "empty_kept_slots": empty}
 
 
+def _density(density_r: torch.Tensor, density_i: Optional[torch.Tensor]):
+    """FP32 densities as the library reads them: two arrays, or (density_i None) one complex array."""
+    if density_i is not None:
+        return _f32(density_r), _f32(density_i)
+    return (density_r.detach().to(torch.complex64).resolve_conj().resolve_neg().contiguous(),)
+
+
+def _density_args(density: torch.Tensor, split: bool = False):
+    """(density_r, density_i) arguments of the autograd functions: a complex density goes in whole, so
+    that neither its parts nor their gradients pass through kernels of their own."""
+    if torch.is_complex(density):
+        return (density.real, density.imag) if split else (density, None)
+    return density, torch.zeros_like(density)
+
+
 class _VoxelizeFn(torch.autograd.Function):
-    """Fused voxelizer: raw Gaussian parameters -> complex64 volume.
+    """Fused voxelizer: raw Gaussian parameters -> complex64 volume.  A
+    complex density comes as density_r with density_i = None.
 
     Forward = TileVoxelizer.forward's preprocess + binning + tile forward
     (reference tile_voxelizer.py:282-309); backward = the tile backward plus
@@ -149,29 +185,36 @@ class _VoxelizeFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, positions, scales, rotations, density_r, density_i, shape, deterministic, tuner=None):
-        params = tuple(_f32(t) for t in (positions, scales, rotations, density_r, density_i))
+        params = (_f32(positions), _f32(scales), _f32(rotations), *_density(density_r, density_i))
         dev = _require_cuda(*params)
         flags = _lib.GSV_BACKWARD_DETERMINISTIC if deterministic else 0
         with torch.cuda.device(dev):
-            plan = prepare_and_bin(params, shape, flags)
-            plan.tuning = tuner.pick(plan, params) if tuner is not None else None
+            prepared = _Prepared(params, shape, flags)
             vol = torch.empty((shape.d, shape.h, shape.w), dtype=torch.complex64, device=dev)
+            plan = prepared.bin()
+            plan.tuning = tuner.pick(plan, params) if tuner is not None else None
             check(lib.gsv_forward_ex(shape, plan.n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.capacity,
-                                     _ptr(vol), _tuning_ref(plan), _stream(dev)), "gsv_forward")
+                                     _ptr(vol), _tuning_ref(plan), prepared.stream), "gsv_forward")
         ctx.plan = plan
-        ctx.save_for_backward(*params)
+        ctx.densities = [(t.shape, t.dtype) for t in params[3:]]  # their values are in the plan's records
+        ctx.save_for_backward(*params[:3])
         return vol
 
     @staticmethod
     def backward(ctx, grad_vol):
-        params = ctx.saved_tensors
-        plan: BinPlan = ctx.plan
-        dev = plan.device
-        g = grad_vol.resolve_conj().to(torch.complex64).contiguous()
-        outs = [torch.empty_like(t) for t in params]
-        with torch.cuda.device(dev):
-            backward_into(plan, params, g, outs)
-        return (*outs, None, None, None)
+        with torch.cuda.device(ctx.plan.device):
+            outs = _backward(ctx, grad_vol)
+        return (*outs, *(None,) * (8 - len(outs)))
+
+
+def _backward(ctx, grad_vol: torch.Tensor):
+    """Gradients of the parameters for an upstream volume gradient."""
+    params = ctx.saved_tensors
+    g = grad_vol.resolve_conj().to(torch.complex64).contiguous()
+    outs = [torch.empty_like(t) for t in params]
+    outs += [torch.empty(shape, dtype=dtype, device=params[0].device) for shape, dtype in ctx.densities]
+    backward_into(ctx.plan, params, g, outs)
+    return outs
 
 
 def _tuning_ref(plan):
@@ -180,12 +223,12 @@ def _tuning_ref(plan):
 
 
 def backward_into(plan: BinPlan, params, grad_vol: torch.Tensor, outs) -> None:
-    pos, scl, rot, dr, di = params
-    gp = GsvParams(pos.data_ptr(), scl.data_ptr(), rot.data_ptr(), dr.data_ptr(), di.data_ptr(), plan.n)
-    gg = GsvGrads(*(o.data_ptr() for o in outs))
-    check(lib.gsv_backward_ex(ctypes.byref(gp), plan.shape, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs),
-                              plan.capacity, _ptr(grad_vol), ctypes.byref(gg), plan.flags, _tuning_ref(plan),
-                              _stream(plan.device)), "gsv_backward")
+    pp, _ = _pointers(params)
+    go, stride = _pointers(outs)
+    gp, gg = GsvParams(*pp, plan.n), GsvGrads(*go)
+    check(lib.gsv_backward_strided(ctypes.byref(gp), plan.shape, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs),
+                                   plan.capacity, _ptr(grad_vol), ctypes.byref(gg), stride, plan.flags,
+                                   _tuning_ref(plan), _stream(plan.device)), "gsv_backward")
 
 
 class StaticPlan(BinPlan):
@@ -218,34 +261,30 @@ class _VoxelizeStaticFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, positions, scales, rotations, density_r, density_i, plan):
-        params = tuple(_f32(t) for t in (positions, scales, rotations, density_r, density_i))
+        params = (_f32(positions), _f32(scales), _f32(rotations), *_density(density_r, density_i))
         dev = plan.device
         if int(params[0].shape[0]) != plan.n:
             raise ValueError(f"static plan is sized for {plan.n} Gaussians, got {int(params[0].shape[0])}")
         st = _stream(dev)
-        gp = GsvParams(*(t.data_ptr() for t in params), plan.n)
-        if plan.live is None:
-            check(lib.gsv_prepare(ctypes.byref(gp), plan.shape, _ptr(plan.ws_gauss), plan.gauss_bytes, None, st),
-                  "gsv_prepare")
-        else:
-            check(lib.gsv_prepare_live(ctypes.byref(gp), _ptr(plan.live), plan.shape, _ptr(plan.ws_gauss),
-                                       plan.gauss_bytes, None, st), "gsv_prepare_live")
+        ptrs, stride = _pointers(params)
+        gp = GsvParams(*ptrs, plan.n)
+        live = _ptr(plan.live) if plan.live is not None else None
+        check(lib.gsv_prepare_strided(ctypes.byref(gp), stride, live, plan.shape, _ptr(plan.ws_gauss),
+                                      plan.gauss_bytes, None, None, st), "gsv_prepare")
         check(lib.gsv_bin(plan.shape, plan.n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.pair_bytes,
                           plan.capacity, st), "gsv_bin")
         vol = torch.empty((plan.shape.d, plan.shape.h, plan.shape.w), dtype=torch.complex64, device=dev)
         check(lib.gsv_forward(plan.shape, plan.n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.capacity,
                               _ptr(vol), st), "gsv_forward")
         ctx.plan = plan
-        ctx.save_for_backward(*params)
+        ctx.densities = [(t.shape, t.dtype) for t in params[3:]]
+        ctx.save_for_backward(*params[:3])
         return vol
 
     @staticmethod
     def backward(ctx, grad_vol):
-        params = ctx.saved_tensors
-        g = grad_vol.resolve_conj().to(torch.complex64).contiguous()
-        outs = [torch.empty_like(t) for t in params]
-        backward_into(ctx.plan, params, g, outs)
-        return (*outs, None)
+        outs = _backward(ctx, grad_vol)
+        return (*outs, *(None,) * (6 - len(outs)))
 
 
 def voxelize(positions: torch.Tensor, scales: torch.Tensor, rotations: torch.Tensor,
@@ -370,11 +409,8 @@ class TileVoxelizer(nn.Module):
     def forward(self, positions: torch.Tensor, scales: torch.Tensor, rotations: torch.Tensor,
                 density: torch.Tensor, chunk_size: int = 4096) -> torch.Tensor:
         del chunk_size
-        if torch.is_complex(density):
-            dr, di = density.real, density.imag
-        else:
-            dr, di = density, torch.zeros_like(density)
-        return _VoxelizeFn.apply(positions, scales, rotations, dr, di, self._shape, self.deterministic, self.tuner)
+        den = _density_args(density, split=self.tuner is not None)  # the tuner times the two-array form
+        return _VoxelizeFn.apply(positions, scales, rotations, *den, self._shape, self.deterministic, self.tuner)
 
     def static(self, n: int, capacity: int, live: Optional[torch.Tensor] = None) -> "StaticVoxelizer":
         """A sync-free, allocation-free variant for `n` Gaussians and at most
@@ -410,11 +446,7 @@ class StaticVoxelizer:
         self.plan = plan
 
     def __call__(self, positions, scales, rotations, density, chunk_size: int = 4096):
-        if torch.is_complex(density):
-            dr, di = density.real, density.imag
-        else:
-            dr, di = density, torch.zeros_like(density)
-        return _VoxelizeStaticFn.apply(positions, scales, rotations, dr, di, self.plan)
+        return _VoxelizeStaticFn.apply(positions, scales, rotations, *_density_args(density), self.plan)
 
 
 def num_tiles(volume_shape, tile_size: int) -> int:

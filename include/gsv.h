@@ -127,6 +127,14 @@ GSV_API int gsv_prepare(const gsv_params* params, gsv_shape shape, void* ws_gaus
 GSV_API int gsv_prepare_live(const gsv_params* params, const int32_t* live, gsv_shape shape, void* ws_gauss,
                              size_t ws_gauss_bytes, int64_t* total_pairs_host, void* stream);
 
+/* gsv_prepare / gsv_prepare_live (live may be NULL) with densities
+ * `density_stride` floats apart: 2 reads an interleaved complex array
+ * (density_i = density_r + 1) where it lies.  With `total_pairs_host` the
+ * status bits come back in the same copy (flags_host may be NULL). */
+GSV_API int gsv_prepare_strided(const gsv_params* params, int64_t density_stride, const int32_t* live,
+                                gsv_shape shape, void* ws_gauss, size_t ws_gauss_bytes,
+                                int64_t* total_pairs_host, int32_t* flags_host, void* stream);
+
 /* Sort the (tile, Gaussian) pairs of the last gsv_prepare / gsv_prepare_live
  * on this workspace by tile (stable: ascending Gaussian id within a tile)
  * and build the per-tile ranges.  If the pair total exceeds `capacity` only
@@ -229,6 +237,11 @@ GSV_API int gsv_forward_ex(gsv_shape shape, int64_t n, const void* ws_gauss, con
 GSV_API int gsv_backward_ex(const gsv_params* params, gsv_shape shape, void* ws_gauss, void* ws_pairs,
                             int64_t capacity, const float* grad_volume, const gsv_grads* grads, int flags,
                             const gsv_tuning* tuning, void* stream);
+/* gsv_backward_ex with the density gradients `density_stride` floats apart
+ * (2: an interleaved complex array, density_i = density_r + 1). */
+GSV_API int gsv_backward_strided(const gsv_params* params, gsv_shape shape, void* ws_gauss, void* ws_pairs,
+                                 int64_t capacity, const float* grad_volume, const gsv_grads* grads,
+                                 int64_t density_stride, int flags, const gsv_tuning* tuning, void* stream);
 
 /* No counterpart in the reference: a census of the work the tile-8 render
  * kernels do on a binned problem (a diagnostic for the roofline; results
