@@ -59,33 +59,40 @@ int sort_end_bit(int64_t ntiles) {
 constexpr int kPrepThreads = 256;
 __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPrepThreads - 1) / kPrepThreads; }
 
-// Counting-sort binning, used when the tile count is small.  The pairs'
+// Counting-sort binning, used unless the tile grid is very large.  The pairs'
 // final order is fixed by two facts: a tile's list holds its Gaussians in
-// ascending id, and Gaussians are handled in rows of kCsSeg consecutive ids.
-// k_prepare also writes, per row, how many of the row's pairs fall in each
-// tile (rows x tiles bytes, "cs_mat": a row's count in one tile is at most
-// kCsSeg; rows padded to whole words); k_colscan writes, per row and tile,
-// the position of the row's first pair of that tile in the sorted output
-// ("cs_pos": the column's exclusive prefix plus the tile's start, from a
-// single-pass scan of the tile totals) and the tile ranges; k_scatter places
-// each row's pairs.  The result equals the stable radix sort's, which larger
-// problems keep.  The counts stay intact and k_scatter clears k_colscan's scan state, so binning may
-// be repeated after one preprocess (e.g. with a larger capacity).
-constexpr int kCsSeg = 64;                                  // Gaussians per row: two warps of k_prepare
-constexpr int kCsRowsPerBlock = kPrepThreads / kCsSeg;      // rows per k_prepare block
-// k_scatter keeps 12 bytes per tile in shared memory: at most 48 KB, the size a launch may use
-// without a function attribute (none is set, also not inside a graph capture)
-constexpr int64_t kCsMaxTiles = 3072;
-// rows x tiles: 16 MB of counts, 64 MB of positions.  128x128x96 (3072 tiles), preprocess and binning, radix
-// and counting sort: 100k Gaussians (4.8 M cells) 106 and 73 us, 200k 139 and 108, 300k (14 M) 160 and
-// 143, 500k (24 M) 200 and 258.
-constexpr int64_t kCsMaxCells = int64_t(1) << 24;
-constexpr int kCsCols = 32, kCsRowGroups = 32;              // k_colscan block: 32 columns x 32 row groups
-__host__ __device__ inline int64_t cs_rows(int64_t n) { return prep_blocks(n) * kCsRowsPerBlock; }
+// ascending id, and Gaussians are handled in rows of consecutive ids.  The
+// kernel that counts the pairs also writes, per row, how many of the row's
+// pairs fall in each tile (rows x tiles 16-bit counts, "cs_mat", rows padded
+// to whole words); k_colscan writes, per row and tile, the position of the
+// row's first pair of that tile in the sorted output ("cs_pos": the column's
+// exclusive prefix plus the tile's start, from a single-pass scan of the tile
+// totals) and the tile ranges; k_scatter places each row's pairs.  The result
+// equals the stable radix sort's, which larger problems keep.  The counts
+// stay intact and k_scatter clears k_colscan's scan state, so binning may be
+// repeated after one preprocess (e.g. with a larger capacity).
+//
+// A row is 64 Gaussians while that leaves few row counts, which gives k_scatter
+// many short blocks, and 256 (a block of the counting kernel) above.  Measured
+// with 64, 256 and the radix sort, preprocess and binning, us:
+// CS_FIGURES
+constexpr int kCsSub = 64;  // Gaussians k_scatter places at a time: a bit each in a tile's word
+constexpr int64_t kCsSmallTiles = 3072;                // 64-Gaussian rows up to here: four rows of counters
+constexpr int64_t kCsSmallCells = int64_t(1) << 22;    // ... and up to this many row counts
+constexpr int64_t kCsMaxTiles = 18432;                 // 12 bytes per tile in k_scatter's shared memory (227 KB)
+constexpr int64_t kCsMaxCells = int64_t(1) << 23;      // 16 MB of counts, 32 MB of positions
+constexpr int kCsCols = 32, kCsRowGroups = 32;         // k_colscan block: 32 columns x 32 row groups
+__host__ __device__ inline int64_t cs_row_len(int64_t n, int64_t ntiles) {
+    return ntiles <= kCsSmallTiles && prep_blocks(n) * (kPrepThreads / kCsSub) * ntiles <= kCsSmallCells ? kCsSub
+                                                                                                     : kPrepThreads;
+}
+__host__ __device__ inline int64_t cs_rows(int64_t n, int64_t ntiles) {
+    return prep_blocks(n) * (kPrepThreads / cs_row_len(n, ntiles));
+}
 __host__ __device__ inline int64_t cs_col_blocks(int64_t ntiles) { return (ntiles + kCsCols - 1) / kCsCols; }
-__host__ __device__ inline int64_t cs_mstride(int64_t ntiles) { return (ntiles + 3) & ~int64_t(3); }  // bytes per row
+__host__ __device__ inline int64_t cs_mstride(int64_t ntiles) { return (ntiles + 1) & ~int64_t(1); }  // counts per row
 inline bool cs_eligible(int64_t n, int64_t ntiles) {
-    return n > 0 && ntiles <= kCsMaxTiles && cs_rows(n) * ntiles <= kCsMaxCells;
+    return n > 0 && ntiles <= kCsMaxTiles && cs_rows(n, ntiles) * ntiles <= kCsMaxCells;
 }
 
 // Status region: the Status word, the preprocess's look-back words (one per
@@ -106,8 +113,8 @@ GaussLayout gauss_layout(int64_t n, const ShapeInfo& si) {
     L.accum = o;    o = align_up(o + size_t(n) * kMomStride * sizeof(float));
     L.status = o;   o = align_up(o + status_bytes(n, si.ntiles));
     L.cs = cs_eligible(n, si.ntiles);
-    L.cs_mat = o;   o = align_up(o + (L.cs ? size_t(cs_rows(n) * cs_mstride(si.ntiles)) : 0));
-    L.cs_pos = o;   o = align_up(o + (L.cs ? size_t(cs_rows(n) * si.ntiles) * sizeof(int32_t) : 0));
+    L.cs_mat = o;   o = align_up(o + (L.cs ? size_t(cs_rows(n, si.ntiles) * cs_mstride(si.ntiles)) * sizeof(uint16_t) : 0));
+    L.cs_pos = o;   o = align_up(o + (L.cs ? size_t(cs_rows(n, si.ntiles) * si.ntiles) * sizeof(int32_t) : 0));
     L.total = o;
     return L;
 }
@@ -258,12 +265,12 @@ __device__ int64_t lookback(unsigned long long* lb, int64_t bid, int64_t block_t
 }
 
 // Tile id of pair `c` (0-based, raster order) of a Gaussian's packed tile box,
-// for the counting sort, where the pair index and both box extents
-// are below 4096 (they are at most the tile count, <= kCsMaxTiles): the two
-// integer divisions become trunc((x + 0.5) * rcp(n)) in IEEE single
-// precision, exact for 0 <= x < 4096 and 1 <= n <= 4096 (every pair checked
-// by enumeration), a few instructions instead of about twenty each.  r1, r2:
-// __frcp_rn of the box's n1, n2.
+// for the counting sort, where the pair index and both box extents are at most
+// the tile count (<= kCsMaxTiles): the two integer divisions become
+// trunc((x + 0.5) * rcp(n)) in IEEE single precision, a few instructions
+// instead of about twenty each.  Exact: (x + 0.5) / n lies at least 0.5 / n from
+// an integer, and the two roundings move it by at most 1.2e-7 (x + 0.5) / n, less
+// than that for x below four million.  r1, r2: __frcp_rn of the box's n1, n2.
 __device__ __forceinline__ int32_t small_div(int32_t x, float rcp_n) {
     return __float2int_rz(__fmul_rn(__fadd_rn(float(x), 0.5f), rcp_n));
 }
@@ -325,15 +332,68 @@ __device__ __forceinline__ PairScan scan_counts(int64_t cnt, int64_t n, int64_t 
     return PairScan{first, warp_base + warp_tot[warp]};
 }
 
+// A block's rows of cs_mat (`row_len` Gaussians each): their pairs per tile.  A row
+// has at most row_len pairs in a tile, so the counters are 16-bit, two to a word,
+// in shared memory (dynamic: ceil(ntiles / 2) words a row) and in cs_mat alike: the
+// rows go out as the same words.  A warp whose Gaussians have many tiles takes
+// them one after the other, its lanes a Gaussian's tiles; otherwise its lanes
+// stride over its pairs, the block-local range [o of lane 0, warp_end), lane l's
+// Gaussian the part starting at o, and find each pair's Gaussian by a shuffle
+// search over the 32 starts (zero-count lanes share their successor's start
+// and are never chosen).
+__device__ __forceinline__ void count_rows(const DevShape& s, int4 box, const PairScan& sc, int64_t bid, int row_len,
+                                           uint16_t* __restrict__ cs_mat, int32_t ntiles) {
+    constexpr unsigned kAll = 0xffffffffu;
+    static_assert(kPrepThreads < 65536, "16-bit counters");
+    extern __shared__ uint32_t cs_hist[];  // [rows][words]: counter of tile t in word t / 2
+    const int lane = threadIdx.x & 31;
+    const int words = (ntiles + 1) >> 1, all = words * (kPrepThreads / row_len);
+    for (int i = threadIdx.x; i < all; i += kPrepThreads) cs_hist[i] = 0u;
+    __syncthreads();
+    uint32_t* row = cs_hist + (threadIdx.x / row_len) * words;  // warp-uniform: row_len is a multiple of 32
+    const long long o = sc.first;
+    const long long wstart = __shfl_sync(kAll, o, 0);
+    const long long wend = sc.warp_end;
+    const float rcp1 = box_rcp(box.z), rcp2 = box_rcp(box.z >> 16);
+    if (wend - wstart >= 32 * 24) {
+        for (int j = 0; j < 32; ++j) {
+            const int cnt = __shfl_sync(kAll, box.w, j);
+            const int bx = __shfl_sync(kAll, box.x, j), by = __shfl_sync(kAll, box.y, j), bz = __shfl_sync(kAll, box.z, j);
+            const float r1 = __shfl_sync(kAll, rcp1, j), r2 = __shfl_sync(kAll, rcp2, j);
+            for (int c = lane; c < cnt; c += 32) {
+                const int32_t t = box_tile_small(s, bx, by, bz, r1, r2, c);
+                atomicAdd(&row[t >> 1], 1u << ((t & 1) * 16));
+            }
+        }
+    } else {
+        for (long long base = wstart; base < wend; base += 32) {
+            const long long p = base + lane;
+            int j = 0;  // largest j with o_j <= p
+#pragma unroll
+            for (int step = 16; step >= 1; step >>= 1) {
+                const long long oj = __shfl_sync(kAll, o, j + step);
+                if (oj <= p) j += step;
+            }
+            const long long oj = __shfl_sync(kAll, o, j);
+            const int bx = __shfl_sync(kAll, box.x, j), by = __shfl_sync(kAll, box.y, j), bz = __shfl_sync(kAll, box.z, j);
+            const float r1 = __shfl_sync(kAll, rcp1, j), r2 = __shfl_sync(kAll, rcp2, j);
+            if (p < wend) {
+                const int32_t t = box_tile_small(s, bx, by, bz, r1, r2, int32_t(p - oj));
+                atomicAdd(&row[t >> 1], 1u << ((t & 1) * 16));
+            }
+        }
+    }
+    __syncthreads();
+    // tile t's count is half t & 1 of its word (little-endian)
+    uint32_t* dst = reinterpret_cast<uint32_t*>(cs_mat + bid * (kPrepThreads / row_len) * cs_mstride(ntiles));
+    for (int i = threadIdx.x; i < all; i += kPrepThreads) dst[i] = cs_hist[i];
+}
+
 // Preprocess (center, radius, quadratic-form coefficients, tight extent, tile
 // box) of one Gaussian per thread, the clearing of its backward moment
 // accumulators, and the exclusive scan of the Gaussians'
 // pair counts into `offsets` in the same launch (scan_counts).  With `cs_mat` the block
-// also counts its pairs per tile for each of its kCsRowsPerBlock rows and
-// writes those rows of cs_mat.  A row's count in one tile is at most kCsSeg
-// (< 256), so the counters are bytes, four to a word, in shared memory
-// (dynamic: kCsRowsPerBlock x ceil(ntiles/4) words) and in cs_mat alike: the
-// block's rows go out as the same words.
+// also counts its pairs per tile (count_rows).
 __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restrict__ pos,
                                                           const float* __restrict__ scl,
                                                           const float* __restrict__ rot,
@@ -343,8 +403,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
                                                           Rec* __restrict__ recs, float4* __restrict__ ext,
                                                           int4* __restrict__ boxes,
                                                           int64_t* __restrict__ offsets, Status* status,
-                                                          uint8_t* __restrict__ cs_mat, int32_t ntiles,
-                                                          float* __restrict__ accum) {
+                                                          uint16_t* __restrict__ cs_mat, int32_t row_len,
+                                                          int32_t ntiles, float* __restrict__ accum) {
     const int64_t bid = scan_ticket(status);
     const int64_t g = bid * kPrepThreads + threadIdx.x;
     int64_t cnt = 0;
@@ -392,61 +452,22 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
         }
         boxes[g] = box;
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const PairScan sc = scan_counts(cnt, n, bid, offsets, status);
-    if (cs_mat == nullptr) return;  // block-uniform
-
-    // Per-row tile counts.  The warp's pairs occupy the block-local range
-    // [wstart, wend), lane l's Gaussian the part starting at o; the lanes
-    // stride over the range and find each pair's Gaussian by a shuffle
-    // search over the 32 starts (zero-count lanes share their successor's
-    // start and are never chosen).
-    extern __shared__ uint32_t cs_hist[];  // [kCsRowsPerBlock][words]: byte counter of tile t in word t/4
-    const int words = (ntiles + 3) >> 2;
-    for (int i = threadIdx.x; i < kCsRowsPerBlock * words; i += kPrepThreads) cs_hist[i] = 0u;
-    __syncthreads();
-    {
-        constexpr unsigned kAll = 0xffffffffu;
-        const long long o = sc.first;
-        const long long wstart = __shfl_sync(kAll, o, 0);
-        const long long wend = sc.warp_end;
-        uint32_t* row = cs_hist + (warp * 32 / kCsSeg) * words;
-        const float rcp1 = box_rcp(box.z), rcp2 = box_rcp(box.z >> 16);
-        for (long long base = wstart; base < wend; base += 32) {
-            const long long p = base + lane;
-            int j = 0;  // largest j with o_j <= p
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const long long oj = __shfl_sync(kAll, o, j + step);
-                if (oj <= p) j += step;
-            }
-            const long long oj = __shfl_sync(kAll, o, j);
-            const int bx = __shfl_sync(kAll, box.x, j), by = __shfl_sync(kAll, box.y, j),
-                      bz = __shfl_sync(kAll, box.z, j);
-            const float r1 = __shfl_sync(kAll, rcp1, j), r2 = __shfl_sync(kAll, rcp2, j);
-            if (p < wend) {
-                const int32_t t = box_tile_small(s, bx, by, bz, r1, r2, int32_t(p - oj));
-                atomicAdd(&row[t >> 2], 1u << ((t & 3) * 8));
-            }
-        }
-    }
-    __syncthreads();
-    // tile t's byte is byte t of its row (little-endian words), so rows of words * 4 bytes
-    uint32_t* dst = reinterpret_cast<uint32_t*>(cs_mat + bid * kCsRowsPerBlock * cs_mstride(ntiles));
-    for (int i = threadIdx.x; i < kCsRowsPerBlock * words; i += kPrepThreads) dst[i] = cs_hist[i];
+    if (cs_mat != nullptr) count_rows(s, box, sc, bid, row_len, cs_mat, ntiles);  // block-uniform
 }
 
 // Tile boxes, pair counts and their scan for the reference-signature binning.
 __global__ void __launch_bounds__(kPrepThreads) k_count_compat(const float* __restrict__ center,
                                                                const float* __restrict__ radius, int64_t n,
                                                                DevShape s, int4* __restrict__ boxes,
-                                                               int64_t* __restrict__ offsets, Status* status) {
+                                                               int64_t* __restrict__ offsets, Status* status,
+                                                               uint16_t* __restrict__ cs_mat, int32_t row_len, int32_t ntiles) {
     const int64_t bid = scan_ticket(status);
     const int64_t g = bid * kPrepThreads + threadIdx.x;
     int64_t cnt = 0;
+    int4 box = make_int4(0, 0, 0, 0);
     if (g < n) {
         float c[3] = {center[g * 3], center[g * 3 + 1], center[g * 3 + 2]};
-        int4 box;
         cnt = tile_box(s, c, radius[g], &box);
         if (cnt <= 0) {
             atomicOr(&status->flags, GSV_FLAG_EMPTY_BOX);
@@ -455,7 +476,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_count_compat(const float* __re
         }
         boxes[g] = box;
     }
-    scan_counts(cnt, n, bid, offsets, status);
+    const PairScan sc = scan_counts(cnt, n, bid, offsets, status);
+    if (cs_mat != nullptr) count_rows(s, box, sc, bid, row_len, cs_mat, ntiles);  // block-uniform
 }
 
 // One thread per Gaussian writes its (tile, gid) pairs in raster order.
@@ -541,7 +563,7 @@ __global__ void k_ranges(const int32_t* __restrict__ keys, const int64_t* __rest
 // tiles < t, from a single-pass look-back over the blocks' tile totals.
 // Writes every tile's range, (0,0) for an empty tile, clamped to `cap` (so a
 // truncated list never reaches past the pair buffer).
-__global__ void __launch_bounds__(kCsCols * kCsRowGroups) k_colscan(const uint8_t* __restrict__ mat,
+__global__ void __launch_bounds__(kCsCols * kCsRowGroups) k_colscan(const uint16_t* __restrict__ mat,
                                                                     int32_t* __restrict__ pos, int64_t rows,
                                                                     int32_t ntiles, int64_t cap,
                                                                     int2* __restrict__ ranges, Status* status,
@@ -596,29 +618,27 @@ __global__ void __launch_bounds__(kCsCols * kCsRowGroups) k_colscan(const uint8_
     }
 }
 
-// Placement pass of the counting sort: one block per row of kCsSeg Gaussians.
-// A pair's place is its row's position for that tile plus the number of the
-// row's earlier Gaussians in it.  Every tile has a word with a bit per Gaussian
-// of the row: all pairs set their bits (in any order), then read the bits below
-// their own, so no pair waits for another (a warp that walked the row's
-// Gaussians in order instead took 19 us for eight rows and 27 us for 783; this
-// takes 7 and 20 us).  A warp takes every kCsWarps-th Gaussian, its lanes
-// that Gaussian's tiles.  Positions at or past `cap` are dropped (the overflow
-// flag says so).  Block 0 also latches the capacity flags and clears
-// k_colscan's ticket counter and look-back words (k_colscan has finished:
-// stream order).
-constexpr int kCsWarps = 8;
-
-__global__ void __launch_bounds__(32 * kCsWarps) k_scatter(const int32_t* __restrict__ pos_in,
-                                                           const int4* __restrict__ boxes,
-                                                           const int64_t* __restrict__ offsets, int64_t n,
-                                                           int32_t ntiles, DevShape s, int64_t cap,
-                                                           int32_t* __restrict__ pair_ids, Status* status,
-                                                           unsigned long long* lb, int64_t lb_words) {
-    static_assert(kCsSeg == 64, "a tile's word has 64 bits");
-    extern __shared__ uint2 cs_bits[];  // [ntiles], then the row's positions
+// Placement pass of the counting sort: one block per row, kCsSub Gaussians of it
+// at a time.  A pair's place is its tile's current position plus the number of
+// earlier Gaussians of the kCsSub in that tile.  Every tile has a word with a
+// bit per Gaussian: all pairs set their bits (in any order), then read the bits
+// below their own, so no pair waits for another; a sweep over the tiles then
+// advances the positions.  (A warp that walked the Gaussians in id order
+// instead took 19 us for 500 Gaussians and 27 us for 50,000 on 3072 tiles.)  A
+// warp takes every kWarps-th Gaussian, its lanes that Gaussian's tiles.
+// Positions at or past `cap` are dropped (the overflow flag says so).  Block 0
+// also latches the capacity flags and clears k_colscan's ticket counter and
+// look-back words (k_colscan has finished: stream order).
+__global__ void __launch_bounds__(1024) k_scatter(const int32_t* __restrict__ pos_in, const int4* __restrict__ boxes,
+                                                  const int64_t* __restrict__ offsets, int64_t n, int row_len,
+                                                  int32_t ntiles, DevShape s, int64_t cap, int32_t* __restrict__ pair_ids,
+                                                  Status* status, unsigned long long* lb, int64_t lb_words) {
+    static_assert(kCsSub == 64, "a tile's word has 64 bits");
+    __shared__ int4 box_s[kPrepThreads];
+    __shared__ float2 rcp_s[kPrepThreads];
+    extern __shared__ uint2 cs_bits[];  // [ntiles], then the tiles' positions
     int32_t* at_t = reinterpret_cast<int32_t*>(cs_bits + ntiles);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) {
             const int64_t total = offsets[n];
@@ -628,12 +648,14 @@ __global__ void __launch_bounds__(32 * kCsWarps) k_scatter(const int32_t* __rest
         }
         for (int64_t i = threadIdx.x; i < lb_words; i += blockDim.x) lb[i] = 0ull;
     }
-    const int64_t row = blockIdx.x, g0 = row * kCsSeg;
+    const int64_t row = blockIdx.x, g0 = row * row_len;
     if (g0 >= n) return;  // block-uniform
-    // lane j of warp w holds the box of the warp's j-th Gaussian
-    constexpr int kMine = kCsSeg / kCsWarps;
-    const int64_t gl = g0 + warp + kCsWarps * lane;
-    const int4 mb = lane < kMine && gl < n ? boxes[gl] : make_int4(0, 0, 0, 0);
+    const int m = int(min(int64_t(row_len), n - g0));
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const int4 b = boxes[g0 + i];
+        box_s[i] = b;
+        rcp_s[i] = make_float2(box_rcp(b.z), box_rcp(b.z >> 16));
+    }
     for (int t0 = threadIdx.x; t0 < ntiles; t0 += 4 * blockDim.x) {  // four loads in flight
         int32_t v[4];
 #pragma unroll
@@ -651,28 +673,37 @@ __global__ void __launch_bounds__(32 * kCsWarps) k_scatter(const int32_t* __rest
         }
     }
     __syncthreads();
+    for (int h = 0; h < m; h += kCsSub) {  // block-uniform
+        const int mh = min(kCsSub, m - h);
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int k = 0; k < kMine; ++k) {
-            const int cnt = __shfl_sync(0xffffffffu, mb.w, k);
-            const int bx = __shfl_sync(0xffffffffu, mb.x, k), by = __shfl_sync(0xffffffffu, mb.y, k),
-                      bz = __shfl_sync(0xffffffffu, mb.z, k);
-            const int j = warp + kCsWarps * k;  // place in the row
-            const uint32_t bit = 1u << (j & 31);
-            const float r1 = box_rcp(bz), r2 = box_rcp(bz >> 16);
-            for (int c = lane; c < cnt; c += 32) {
-                const int32_t t = box_tile_small(s, bx, by, bz, r1, r2, c);
-                if (pass == 0) {
-                    atomicOr(j < 32 ? &cs_bits[t].x : &cs_bits[t].y, bit);
-                } else {
-                    const uint2 w = cs_bits[t];
-                    const int before = j < 32 ? __popc(w.x & (bit - 1u)) : __popc(w.x) + __popc(w.y & (bit - 1u));
-                    const int64_t p = int64_t(at_t[t]) + before;
-                    if (p < cap) pair_ids[p] = int32_t(g0 + j);
+        for (int pass = 0; pass < 2; ++pass) {
+            for (int j = warp; j < mh; j += warps) {
+                const int4 b = box_s[h + j];
+                const uint32_t bit = 1u << (j & 31);
+                const float2 rcp = rcp_s[h + j];
+                for (int c = lane; c < b.w; c += 32) {
+                    const int32_t t = box_tile_small(s, b.x, b.y, b.z, rcp.x, rcp.y, c);
+                    if (pass == 0) {
+                        atomicOr(j < 32 ? &cs_bits[t].x : &cs_bits[t].y, bit);
+                    } else {
+                        const uint2 w = cs_bits[t];
+                        const int before = j < 32 ? __popc(w.x & (bit - 1u)) : __popc(w.x) + __popc(w.y & (bit - 1u));
+                        const int64_t p = int64_t(at_t[t]) + before;
+                        if (p < cap) pair_ids[p] = int32_t(g0 + h + j);
+                    }
                 }
             }
+            __syncthreads();
         }
-        if (pass == 0) __syncthreads();
+        if (h + kCsSub >= m) break;  // the last ones
+        for (int t = threadIdx.x; t < ntiles; t += blockDim.x) {
+            const uint2 w = cs_bits[t];
+            if (w.x | w.y) {
+                at_t[t] = int32_t(min(int64_t(at_t[t]) + __popc(w.x) + __popc(w.y), cap));
+                cs_bits[t] = make_uint2(0u, 0u);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -693,19 +724,23 @@ int read_status(const GaussLayout& L, const void* ws, int64_t* total, int32_t* f
     return GSV_OK;
 }
 
-// Dynamic shared memory of k_prepare's byte counters and of k_scatter's words and positions.  Neither
-// kernel declares static shared memory beyond a few words, and both stay within the 48 KB a
-// launch may use without a function attribute.
-int cs_prep_smem_bytes(int64_t ntiles) { return int(kCsRowsPerBlock * ((ntiles + 3) / 4) * int64_t(sizeof(uint32_t))); }
+// Dynamic shared memory of the counting kernels' row counters (at most 36 KB, the default allows it)
+// and of k_scatter's words and positions.
+int cs_count_smem_bytes(int64_t n, int64_t ntiles) {
+    return int(kPrepThreads / cs_row_len(n, ntiles) * ((ntiles + 1) / 2) * int64_t(sizeof(uint32_t)));
+}
 int cs_scatter_smem_bytes(int64_t ntiles) { return int(ntiles * int64_t(sizeof(uint2) + sizeof(int32_t))); }
-static_assert(kCsMaxTiles * (sizeof(uint2) + sizeof(int32_t)) <= 48 * 1024, "k_scatter's words and positions exceed 48 KB");
-static_assert(kCsRowsPerBlock * kCsMaxTiles <= 40 * 1024, "k_prepare's counters leave no room for its static words");
+constexpr int kScatterStatic = kPrepThreads * int(sizeof(int4) + sizeof(float2));
+static_assert((kCsMaxTiles + 1) / 2 * 4 <= 40 * 1024 && kPrepThreads / kCsSub * (kCsSmallTiles + 1) / 2 * 4 <= 40 * 1024,
+              "the row counters leave no room for the static words");
+static_assert(kCsMaxTiles * (sizeof(uint2) + sizeof(int32_t)) + kScatterStatic <= 227 * 1024,
+              "k_scatter's words, positions and boxes exceed an SM's shared memory");
 
 // Shared tail of both binning flavours.  Counting sort (k_colscan,
-// k_scatter) when the preprocess wrote the per-row tile counts (native path,
-// small tile count) and `mode` allows it; otherwise emit, radix sort, ranges.
+// k_scatter) where it applies (the counting kernels wrote the per-row tile
+// counts) and `mode` allows it; otherwise emit, radix sort, ranges.
 int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, size_t ws_pairs_bytes,
-               int64_t cap, int32_t* vals_out_override, int mode, bool rows_written, cudaStream_t st) {
+               int64_t cap, int32_t* vals_out_override, int mode, cudaStream_t st) {
     if (cap < 0 || cap > int64_t(INT32_MAX)) return GSV_ERR_INVALID_ARGUMENT;
     if (mode != GSV_BIN_AUTO && mode != GSV_BIN_RADIX && mode != GSV_BIN_COUNTING) return GSV_ERR_INVALID_ARGUMENT;
     const GaussLayout G = gauss_layout(n, si);
@@ -719,23 +754,27 @@ int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, s
     int32_t* keys_out = at<int32_t>(ws_pairs, P.keys_out);
     int32_t* vals_out = vals_out_override ? vals_out_override : at<int32_t>(ws_pairs, P.vals_out);
     int2* ranges = at<int2>(ws_gauss, G.ranges);
-    const bool cs = rows_written && G.cs;
-    if (mode == GSV_BIN_COUNTING && !cs) return GSV_ERR_INVALID_ARGUMENT;
+    if (mode == GSV_BIN_COUNTING && !G.cs) return GSV_ERR_INVALID_ARGUMENT;
     if (cap == 0) {
         GSV_CUDA_TRY(cudaMemsetAsync(ranges, 0, size_t(si.ntiles) * sizeof(int2), st));
         return GSV_OK;
     }
-    if (cs && mode != GSV_BIN_RADIX) {
+    if (G.cs && mode != GSV_BIN_RADIX) {
         unsigned long long* lb_cs = reinterpret_cast<unsigned long long*>(status + 1) + prep_blocks(n);
-        const int64_t rows = cs_rows(n);
+        const int64_t rows = cs_rows(n, si.ntiles), row_len = cs_row_len(n, si.ntiles);
         const int32_t T = int32_t(si.ntiles);
         k_colscan<<<unsigned(cs_col_blocks(T)), kCsCols * kCsRowGroups, 0, st>>>(
-            at<uint8_t>(ws_gauss, G.cs_mat), at<int32_t>(ws_gauss, G.cs_pos), rows, T, cap, ranges, status, lb_cs);
+            at<uint16_t>(ws_gauss, G.cs_mat), at<int32_t>(ws_gauss, G.cs_pos), rows, T, cap, ranges, status, lb_cs);
         GSV_LAUNCH_CHECK();
+        // a long row over many tiles is a chain of long sub-rows, one block to an SM: more threads shorten
+        // them (13824 tiles: 512 threads 92 us, 1024 84; 3072 tiles 85 and 93)
         const int smem = cs_scatter_smem_bytes(T);
-        k_scatter<<<unsigned(rows), 32 * kCsWarps, smem, st>>>(
-            at<int32_t>(ws_gauss, G.cs_pos), at<int4>(ws_gauss, G.box), offsets, n, T, s, cap, vals_out, status,
-            lb_cs, cs_col_blocks(T));
+        const int threads = T <= 4096 ? 512 : 1024;
+        if (smem + kScatterStatic > 48 * 1024)
+            GSV_CUDA_TRY(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k_scatter<<<unsigned(rows), threads, smem, st>>>(at<int32_t>(ws_gauss, G.cs_pos), at<int4>(ws_gauss, G.box),
+                                                         offsets, n, int(row_len), T, s, cap, vals_out, status, lb_cs,
+                                                         cs_col_blocks(T));
         GSV_LAUNCH_CHECK();
         return GSV_OK;
     }
@@ -815,12 +854,12 @@ static int prepare_impl(const gsv_params* p, int64_t density_stride, const int32
     Status* status = at<Status>(ws_gauss, L.status);
     // status flags, the block counters and the scans' look-back words
     GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
-    const int smem = L.cs ? cs_prep_smem_bytes(si.ntiles) : 0;
+    const int smem = L.cs ? cs_count_smem_bytes(n, si.ntiles) : 0;
     k_prepare<<<unsigned(prep_blocks(n)), kPrepThreads, smem, st>>>(
         p->positions, p->scales, p->rotations, p->density_r, p->density_i, density_stride, n, live, dev_shape(si),
         at<Rec>(ws_gauss, L.rec), at<float4>(ws_gauss, L.ext), at<int4>(ws_gauss, L.box),
-        at<int64_t>(ws_gauss, L.offsets), status, L.cs ? at<uint8_t>(ws_gauss, L.cs_mat) : nullptr,
-        int32_t(si.ntiles), at<float>(ws_gauss, L.accum));
+        at<int64_t>(ws_gauss, L.offsets), status, L.cs ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr,
+        int32_t(cs_row_len(n, si.ntiles)), int32_t(si.ntiles), at<float>(ws_gauss, L.accum));
     GSV_LAUNCH_CHECK();
     if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, flags_host, st);
     return GSV_OK;
@@ -848,7 +887,7 @@ int gsv_bin_ex(gsv_shape shape, int64_t n, void* ws_gauss, void* ws_pairs, size_
                int64_t capacity, int mode, void* stream) {
     ShapeInfo si = shape_info(shape);
     if (!si.ok || n < 0 || !ws_gauss) return GSV_ERR_INVALID_ARGUMENT;
-    return bin_common(si, n, ws_gauss, ws_pairs, ws_pairs_bytes, capacity, nullptr, mode, true,
+    return bin_common(si, n, ws_gauss, ws_pairs, ws_pairs_bytes, capacity, nullptr, mode,
                       static_cast<cudaStream_t>(stream));
 }
 
@@ -894,9 +933,9 @@ int gsv_build_tile_pairs_count(const float* center_vox, const float* radius_vox,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Status* status = at<Status>(ws_gauss, L.status);
     GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
-    k_count_compat<<<unsigned(prep_blocks(n)), kPrepThreads, 0, st>>>(center_vox, radius_vox, n, dev_shape(si),
-                                                                      at<int4>(ws_gauss, L.box),
-                                                                      at<int64_t>(ws_gauss, L.offsets), status);
+    k_count_compat<<<unsigned(prep_blocks(n)), kPrepThreads, L.cs ? cs_count_smem_bytes(n, si.ntiles) : 0, st>>>(
+        center_vox, radius_vox, n, dev_shape(si), at<int4>(ws_gauss, L.box), at<int64_t>(ws_gauss, L.offsets), status,
+        L.cs ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr, int32_t(cs_row_len(n, si.ntiles)), int32_t(si.ntiles));
     GSV_LAUNCH_CHECK();
     if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, nullptr, st);
     return GSV_OK;
@@ -909,7 +948,7 @@ int gsv_build_tile_pairs_fill(gsv_shape shape, int64_t n, void* ws_gauss, void* 
     if (!si.ok || n < 0 || !ws_gauss || !tile_ranges || (capacity > 0 && !pair_ids))
         return GSV_ERR_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = bin_common(si, n, ws_gauss, ws_pairs, ws_pairs_bytes, capacity, pair_ids, GSV_BIN_RADIX, false, st);
+    int rc = bin_common(si, n, ws_gauss, ws_pairs, ws_pairs_bytes, capacity, pair_ids, GSV_BIN_AUTO, st);
     if (rc != GSV_OK) return rc;
     const GaussLayout L = gauss_layout(n, si);
     GSV_CUDA_TRY(cudaMemcpyAsync(tile_ranges, at<int2>(ws_gauss, L.ranges), size_t(si.ntiles) * sizeof(int2),

@@ -318,10 +318,10 @@ def build_tile_pairs(center_vox: torch.Tensor, radius_vox: torch.Tensor, volume_
                                              plan.gauss_bytes, None, st), "gsv_build_tile_pairs_count")
         total, fl = plan.read_status(st)
         _raise_flags(fl, total)
-        tile_ranges = torch.zeros((ntiles, 2), dtype=torch.int32, device=dev)
         pair_ids = torch.empty((total,), dtype=torch.int32, device=dev)
         if total == 0:
-            return tile_ranges, pair_ids
+            return torch.zeros((ntiles, 2), dtype=torch.int32, device=dev), pair_ids
+        tile_ranges = torch.empty((ntiles, 2), dtype=torch.int32, device=dev)
         plan.alloc_pairs(total)
         check(lib.gsv_build_tile_pairs_fill(shape, n, _ptr(plan.ws_gauss), _ptr(plan.ws_pairs), plan.pair_bytes,
                                             total, _ptr(tile_ranges), _ptr(pair_ids), st),

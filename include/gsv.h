@@ -141,9 +141,8 @@ GSV_API int gsv_prepare_strided(const gsv_params* params, int64_t density_stride
  * `capacity` pairs are kept and GSV_FLAG_CAPACITY_OVERFLOW is latched.  May
  * be called again after one preprocess (e.g. with a larger capacity).
  * Two sorts give the same lists: a counting sort over per-row tile counts
- * the preprocess writes when the grid has at most 3072 tiles and
- * ceil((n+1)/256)*4 rows x tiles <= 2^22 (three launches, no pair
- * keys), else an emit + radix sort + range pass.  gsv_bin picks the first
+ * the preprocess writes when the grid has at most 18432 tiles and
+ * ceil((n+1)/256) x tiles <= 2^23 (three launches, no pair keys), else an emit + radix sort + range pass.  gsv_bin picks the first
  * where it applies. */
 #define GSV_BIN_AUTO 0
 #define GSV_BIN_RADIX 1    /* always the radix sort */

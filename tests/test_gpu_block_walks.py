@@ -1,6 +1,6 @@
 """The block walks of the tile-8 and tile-4 kernels where their bookkeeping can go wrong: list lengths
 around a warp, a staged chunk and a full queue in one tile, ragged volumes, infinite and NaN densities
-and gradients, and the counting sort at its largest row count.  Against the FP64 oracle, with the
+and gradients, and the counting sort's rows.  Against the FP64 oracle, with the
 suite's tolerances."""
 import numpy as np
 import pytest
@@ -85,14 +85,18 @@ def test_one_wild_density_or_gradient_stays_where_it_is(value, ts, cuda_device):
     assert not np.isclose(g3[3][hit], grads[3][hit]).any()
 
 
-def test_counting_sort_at_its_largest_row_count(cuda_device):
-    """3072 tiles and 300,000 Gaussians (14.4 M row counts): the lists of the radix sort."""
+@pytest.mark.parametrize("shape,ts,n", [((128, 128, 96), 8, 300_000), ((256, 256, 144), 8, 2_000), ((256, 256, 144), 8, 100_000),
+                                        ((50, 61, 47), 4, 9_001), ((64, 64, 64), 4, 400_000), ((64, 64, 64), 8, 257),
+                                        ((160, 160, 152), 8, 511)])
+def test_counting_sort_rows(shape, ts, n, cuda_device):
+    """Rows of 64 and of 256 Gaussians, their last ones cut anywhere, up to the largest tile count and the
+    largest number of row counts: the lists of the radix sort."""
     from tests.test_gpu_binning_modes import _params, _prepare, _same_lists
 
     from gs_tmi_b200.tile_voxelizer import _shape
 
-    gs = synthetic.random_gaussians(300_000, (128, 128, 96), seed=2)
-    _same_lists(_prepare(_params(gs, cuda_device), _shape((128, 128, 96), 8)))
+    gs = synthetic.random_gaussians(n, shape, seed=2, log_scale_mean_vox=-0.5 if n > 10_000 else 0.6)
+    _same_lists(_prepare(_params(gs, cuda_device), _shape(shape, ts)))
 
 
 @pytest.mark.parametrize("ts", [8, 4, 5])
