@@ -117,6 +117,8 @@ SIGNATURES = {
                                                  ctypes.c_longlong, _vp, _vp]),
     "gsv_sense_workspace_bytes": (_sz, []),
     "gsv_sense_expand": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp]),
+    "gsv_sense_expand_scaled": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp, _vp]),
+    "gsv_sense_adjoint_scaled": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, ctypes.c_float, _vp, _vp]),
     "gsv_sense_residual": (ctypes.c_int, [_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _sz, _vp]),
     "gsv_sense_adjoint": (ctypes.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp]),
     "gsv_tv_magnitude": (ctypes.c_int, [_vp, _i32, _i32, _i32, _vp, _vp, _vp, _sz, _vp]),

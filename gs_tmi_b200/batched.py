@@ -223,16 +223,17 @@ class BatchedRecon:
                 d, h, w = vol.shape
                 nc = self.S[i].shape[0]
                 X = torch.empty_like(self.S[i])
-                check(lib.gsv_sense_expand(vol.data_ptr(), self.S[i].data_ptr(), nc, d, h, w, X.data_ptr(), st),
-                      "gsv_sense_expand")
-                K = torch.fft.fftn(X, dim=(-3, -2, -1), norm="ortho")
+                scale = (d * h * w) ** -0.5  # of the orthonormal transforms, which do not scale themselves
+                check(lib.gsv_sense_expand_scaled(vol.data_ptr(), self.S[i].data_ptr(), nc, d, h, w, scale,
+                                                  X.data_ptr(), st), "gsv_sense_expand")
+                K = torch.fft.fftn(X, dim=(-3, -2, -1), norm="backward")
                 check(lib.gsv_sense_residual(K.data_ptr(), self.mask[i].data_ptr(), self.ku[i].data_ptr(), nc, d,
                                              h, w, self.data_loss[i].data_ptr(), self.ws.data_ptr(), self.ws.numel(),
                                              st), "gsv_sense_residual")
-                G = torch.fft.ifftn(K, dim=(-3, -2, -1), norm="ortho")
+                G = torch.fft.ifftn(K, dim=(-3, -2, -1), norm="forward")
                 gv = sb.grad_volumes[i]
-                check(lib.gsv_sense_adjoint(G.data_ptr(), self.S[i].data_ptr(), nc, d, h, w, gv.data_ptr(), st),
-                      "gsv_sense_adjoint")
+                check(lib.gsv_sense_adjoint_scaled(G.data_ptr(), self.S[i].data_ptr(), nc, d, h, w, scale,
+                                                   gv.data_ptr(), st), "gsv_sense_adjoint")
                 if self.tv_weight > 0:
                     check(lib.gsv_tv_magnitude(vol.data_ptr(), d, h, w, self.tv_loss[i].data_ptr(),
                                                self.tv_grad[i].data_ptr(), self.ws.data_ptr(), self.ws.numel(), st),

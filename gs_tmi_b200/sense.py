@@ -152,8 +152,10 @@ class _SenseDataTerm(torch.autograd.Function):
         nc, (d, h, w) = S.shape[0], vol.shape
         st = torch.cuda.current_stream(vol.device).cuda_stream
         X = torch.empty_like(S)
-        check(lib.gsv_sense_expand(vol.data_ptr(), S.data_ptr(), nc, d, h, w, X.data_ptr(), st), "gsv_sense_expand")
-        K = torch.fft.fftn(X, dim=(-3, -2, -1), norm="ortho")
+        # the orthonormal transforms' factor goes into the coil products: the FFTs do not scale
+        check(lib.gsv_sense_expand_scaled(vol.data_ptr(), S.data_ptr(), nc, d, h, w, (d * h * w) ** -0.5,
+                                          X.data_ptr(), st), "gsv_sense_expand")
+        K = torch.fft.fftn(X, dim=(-3, -2, -1), norm="backward")
         loss = torch.empty((), device=vol.device)
         check(lib.gsv_sense_residual(K.data_ptr(), mask.data_ptr(), ku.data_ptr(), nc, d, h, w, loss.data_ptr(),
                                      ws.data_ptr(), ws.numel(), st), "gsv_sense_residual")
@@ -167,10 +169,11 @@ class _SenseDataTerm(torch.autograd.Function):
         K, S = ctx.saved_tensors
         nc, (d, h, w) = S.shape[0], S.shape[1:]
         with torch.cuda.device(K.device):  # the autograd thread may have no current context
-            G = torch.fft.ifftn(K, dim=(-3, -2, -1), norm="ortho")
+            G = torch.fft.ifftn(K, dim=(-3, -2, -1), norm="forward")
             vg = torch.empty((d, h, w), dtype=torch.complex64, device=K.device)
-            check(lib.gsv_sense_adjoint(G.data_ptr(), S.data_ptr(), nc, d, h, w, vg.data_ptr(),
-                                        torch.cuda.current_stream(K.device).cuda_stream), "gsv_sense_adjoint")
+            check(lib.gsv_sense_adjoint_scaled(G.data_ptr(), S.data_ptr(), nc, d, h, w, (d * h * w) ** -0.5,
+                                               vg.data_ptr(), torch.cuda.current_stream(K.device).cuda_stream),
+                  "gsv_sense_adjoint")
             return vg * gout, None, None, None, None
 
 

@@ -332,6 +332,12 @@ GSV_API int gsv_mlp_gemm_test_timeout(const void* a, const void* b, int M, int N
 GSV_API size_t gsv_sense_workspace_bytes(void);
 GSV_API int gsv_sense_expand(const float* volume, const float* coils, int32_t ncoils, int32_t d, int32_t h, int32_t w,
                              float* out, void* stream);
+/* gsv_sense_expand / gsv_sense_adjoint times `scale` (an orthonormal transform's factor, so that the
+ * transform itself need not scale). */
+GSV_API int gsv_sense_expand_scaled(const float* volume, const float* coils, int32_t ncoils, int32_t d, int32_t h,
+                                    int32_t w, float scale, float* out, void* stream);
+GSV_API int gsv_sense_adjoint_scaled(const float* kgrad_image, const float* coils, int32_t ncoils, int32_t d,
+                                     int32_t h, int32_t w, float scale, float* volume_grad, void* stream);
 GSV_API int gsv_sense_residual(float* kspace, const float* mask, const float* measured, int32_t ncoils, int32_t d,
                                int32_t h, int32_t w, float* loss, void* ws, size_t ws_bytes, void* stream);
 GSV_API int gsv_sense_adjoint(const float* kgrad_image, const float* coils, int32_t ncoils, int32_t d, int32_t h,
