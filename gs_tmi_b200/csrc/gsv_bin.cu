@@ -209,11 +209,11 @@ constexpr int kLbSpinLimit = 1 << 22;  // polls of one predecessor's word before
 
 __device__ __forceinline__ unsigned long long lb_load(const unsigned long long* p) {
     unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void lb_store(unsigned long long* p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Decoupled look-back of scan block `bid`, run by all 32 lanes of one warp:
@@ -227,6 +227,11 @@ __device__ __forceinline__ void lb_store(unsigned long long* p, unsigned long lo
 // has started.  Each retry is bounded: on time-out GSV_FLAG_SCAN_STALLED is
 // latched and the block publishes what it has, so no later block waits the
 // full limit again.
+// A word carries all that is passed on, so it needs no ordering against other
+// accesses: acquire and release, which wait for the block's record stores,
+// cost 50,000 Gaussians 2 us (k_prepare and k_colscan) and 2M 11 us.  Two to
+// eight windows in flight a step measured the same or slower (2M: 172 to 187 us
+// against 161): they only poll more.
 __device__ int64_t lookback(unsigned long long* lb, int64_t bid, int64_t block_tot, Status* status, int lane) {
     if (bid == 0) {
         if (lane == 0) lb_store(&lb[0], kLbPre | (unsigned long long)block_tot);
