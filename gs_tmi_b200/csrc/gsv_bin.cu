@@ -72,19 +72,39 @@ __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPre
 // stay intact and k_scatter clears k_colscan's scan state, so binning may be
 // repeated after one preprocess (e.g. with a larger capacity).
 //
-// A row is 64 Gaussians while that leaves few row counts, which gives k_scatter
-// many short blocks, and 256 (a block of the counting kernel) above.  Measured
-// with 64, 256 and the radix sort, preprocess and binning, us:
-// CS_FIGURES
+// A row is 64 Gaussians, which gives k_scatter many short blocks, while there
+// are no more rows than tiles (a column of k_colscan grows with the rows, a
+// block of k_scatter with the tiles) and few row counts; otherwise 256 (a block
+// of the counting kernel).  Preprocess and binning with rows of 64, of 256 and
+// the radix sort, us:
+//   tiles  Gaussians (pairs each)   64    256   radix
+//     512    20,000 (15)           28.5   30.9   55.4
+//     512    60,000 (11)           40.3   37.3
+//     512   200,000 (6)            65.0   52.7   79.2
+//    1728   120,000 (15)           59.2   56.7
+//    3072    50,000 (36)           48.9   54.6   87.4
+//    3072   200,000 (16)           92.8   79.5  126
+//    3072   500,000 (10)          210    140    182
+//    3072   800,000 (8)                  198    228
+//    3072 1,300,000 (6)                  297    298
+//    9216   154,793 (36)                 130    159
+//    9216   400,000 (20)                 251    224
+//   13824    40,000 (139)                133    179
+//   13824   300,000 (35)                 248    247
+//   18432   230,000 (45)                 253    245
+// k_scatter's lanes per Gaussian, by the row's mean pairs a Gaussian: up to 12 eight, up to 24 sixteen, above a
+// warp.  k_scatter with 8, 16 and 32 lanes, us: 10 pairs 59, 64, 88; 15 pairs 8.1, 7.4, 8.4; 36 pairs 20.6, 17.4,
+// 16.3; 139 pairs 130, 95, 84.
+constexpr int64_t kCsNarrow8 = 12, kCsNarrow16 = 24;
 constexpr int kCsSub = 64;  // Gaussians k_scatter places at a time: a bit each in a tile's word
 constexpr int64_t kCsSmallTiles = 3072;                // 64-Gaussian rows up to here: four rows of counters
 constexpr int64_t kCsSmallCells = int64_t(1) << 22;    // ... and up to this many row counts
 constexpr int64_t kCsMaxTiles = 18432;                 // 12 bytes per tile in k_scatter's shared memory (227 KB)
-constexpr int64_t kCsMaxCells = int64_t(1) << 23;      // 16 MB of counts, 32 MB of positions
+constexpr int64_t kCsMaxCells = int64_t(1) << 23;      // 16 MB of counts, 32 MB of positions; on few tiles twice that
 constexpr int kCsCols = 32, kCsRowGroups = 32;         // k_colscan block: 32 columns x 32 row groups
 __host__ __device__ inline int64_t cs_row_len(int64_t n, int64_t ntiles) {
-    return ntiles <= kCsSmallTiles && prep_blocks(n) * (kPrepThreads / kCsSub) * ntiles <= kCsSmallCells ? kCsSub
-                                                                                                     : kPrepThreads;
+    const int64_t rows = prep_blocks(n) * (kPrepThreads / kCsSub);
+    return ntiles <= kCsSmallTiles && rows <= ntiles && rows * ntiles <= kCsSmallCells ? kCsSub : kPrepThreads;
 }
 __host__ __device__ inline int64_t cs_rows(int64_t n, int64_t ntiles) {
     return prep_blocks(n) * (kPrepThreads / cs_row_len(n, ntiles));
@@ -92,7 +112,8 @@ __host__ __device__ inline int64_t cs_rows(int64_t n, int64_t ntiles) {
 __host__ __device__ inline int64_t cs_col_blocks(int64_t ntiles) { return (ntiles + kCsCols - 1) / kCsCols; }
 __host__ __device__ inline int64_t cs_mstride(int64_t ntiles) { return (ntiles + 1) & ~int64_t(1); }  // counts per row
 inline bool cs_eligible(int64_t n, int64_t ntiles) {
-    return n > 0 && ntiles <= kCsMaxTiles && cs_rows(n, ntiles) * ntiles <= kCsMaxCells;
+    return n > 0 && ntiles <= kCsMaxTiles &&
+           cs_rows(n, ntiles) * ntiles <= (ntiles <= kCsSmallTiles ? 2 * kCsMaxCells : kCsMaxCells);
 }
 
 // Status region: the Status word, the preprocess's look-back words (one per
@@ -660,7 +681,8 @@ __global__ void __launch_bounds__(kCsCols * kCsRowGroups) k_colscan(const uint16
 // below their own, so no pair waits for another; a sweep over the tiles then
 // advances the positions.  (A warp that walked the Gaussians in id order
 // instead took 19 us for 500 Gaussians and 27 us for 50,000 on 3072 tiles.)  A
-// warp takes every kWarps-th Gaussian, its lanes that Gaussian's tiles.
+// group of lanes takes a Gaussian, each lane some of its tiles; how many lanes
+// follows from the row's mean (kCsNarrow8, kCsNarrow16).
 // Positions at or past `cap` are dropped (the overflow flag says so).  Block 0
 // also latches the capacity flags and clears k_colscan's ticket counter and
 // look-back words (k_colscan has finished: stream order).
@@ -673,7 +695,6 @@ __global__ void __launch_bounds__(1024) k_scatter(const int32_t* __restrict__ po
     __shared__ float2 rcp_s[kPrepThreads];
     extern __shared__ uint2 cs_bits[];  // [ntiles], then the tiles' positions
     int32_t* at_t = reinterpret_cast<int32_t*>(cs_bits + ntiles);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) {
             const int64_t total = offsets[n];
@@ -707,16 +728,20 @@ __global__ void __launch_bounds__(1024) k_scatter(const int32_t* __restrict__ po
             }
         }
     }
+    // lanes per Gaussian
+    const int64_t pairs = offsets[g0 + m] - offsets[g0];
+    const int log_g = pairs <= kCsNarrow8 * m ? 3 : pairs <= kCsNarrow16 * m ? 4 : 5;
+    const int slot = threadIdx.x >> log_g, slots = blockDim.x >> log_g, in = threadIdx.x & ((1 << log_g) - 1);
     __syncthreads();
     for (int h = 0; h < m; h += kCsSub) {  // block-uniform
         const int mh = min(kCsSub, m - h);
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
-            for (int j = warp; j < mh; j += warps) {
+            for (int j = slot; j < mh; j += slots) {
                 const int4 b = box_s[h + j];
                 const uint32_t bit = 1u << (j & 31);
                 const float2 rcp = rcp_s[h + j];
-                for (int c = lane; c < b.w; c += 32) {
+                for (int c = in; c < b.w; c += 1 << log_g) {
                     const int32_t t = box_tile_small(s, b.x, b.y, b.z, rcp.x, rcp.y, c);
                     if (pass == 0) {
                         atomicOr(j < 32 ? &cs_bits[t].x : &cs_bits[t].y, bit);

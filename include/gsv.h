@@ -142,7 +142,7 @@ GSV_API int gsv_prepare_strided(const gsv_params* params, int64_t density_stride
  * be called again after one preprocess (e.g. with a larger capacity).
  * Two sorts give the same lists: a counting sort over per-row tile counts
  * the preprocess writes when the grid has at most 18432 tiles and
- * ceil((n+1)/256) x tiles <= 2^23 (three launches, no pair keys), else an emit + radix sort + range pass.  gsv_bin picks the first
+ * ceil((n+1)/256) x tiles <= 2^23, or 2^24 on at most 3072 tiles (three launches, no pair keys), else an emit + radix sort + range pass.  gsv_bin picks the first
  * where it applies. */
 #define GSV_BIN_AUTO 0
 #define GSV_BIN_RADIX 1    /* always the radix sort */
