@@ -20,8 +20,8 @@
 // (the layer's bias gradient).
 // What bounds it: with K = 256 the epilogue's traffic (z and the activation,
 // six bytes an output).  84,375 x 256 x 256: bias + GELU 37 us (4.7 TB/s; 88 us
-// with one tile per CTA and cp.async), GELU' 41 us (116 us), weight gradient
-// 20 us (56 us); at 189,440 rows another 94,720 cost 35 us, 5.5 TB/s.
+// with one tile per CTA and cp.async), GELU' 42 us (116 us), weight gradient
+// 20 us (56 us); at 189,440 rows another 94,720 cost GELU' 35 us, 5.5 TB/s.
 // Every mbarrier wait is bounded; on time-out the kernel latches an error
 // flag, skips the epilogue, waits (bounded) until the tensor-core work and the
 // copies it issued have retired, frees its TMEM and returns.
