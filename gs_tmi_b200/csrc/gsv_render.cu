@@ -157,6 +157,16 @@ __device__ __forceinline__ float warp_reduce_scatter16(float v[16], int lane) {
     return v[0] + __shfl_xor_sync(kFull, v[0], 1);
 }
 
+// Whether a Gaussian's moments add anything.  With none of its voxels included they are all zero, and its
+// coefficients may be NaN or infinite: 0 * NaN must not reach the gradient, which is zero (the reference
+// sums over included voxels only, tile_voxelize_cuda_kernel.cu:217-252).
+__device__ __forceinline__ bool any_moment(const float m[kMom]) {
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < kMom; ++i) any |= m[i] != 0.f;
+    return any;
+}
+
 // Compat outputs for one (tile, Gaussian): every lane holds `tot` (lane 2i
 // holds moment i); lanes 0..13 issue one atomic each.
 __device__ __forceinline__ void compat_emit(const RenderArgs& a, const Rec& g, int gid, float tot,
@@ -164,6 +174,7 @@ __device__ __forceinline__ void compat_emit(const RenderArgs& a, const Rec& g, i
     float m[kMom];
 #pragma unroll
     for (int i = 0; i < kMom; ++i) m[i] = __shfl_sync(kFull, tot, 2 * i);
+    if (!any_moment(m)) return;  // warp-uniform
     float out;
     switch (lane) {
         case 0: out = m[0]; break;
@@ -396,6 +407,7 @@ __device__ __forceinline__ bool needs_guard(const Rec& r) {
 // The moments of one (tile, Gaussian) pair to the gradients of the reference's own parameters.
 __device__ __forceinline__ void compat_emit_lane(const RenderArgs& a, const Rec& g, int gid, const float m[kMomStride],
                                                  const float ih[3]) {
+    if (!any_moment(m)) return;
     atomicAdd(a.g_dr + gid, m[0]);
     atomicAdd(a.g_di + gid, m[1]);
     // dL/dcenter_a = -2 sum_b Q_ab S1_b   (reference: -2 (M d)_a / hs_a, .cu:241-243)
