@@ -830,8 +830,11 @@ int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, s
         // them (13824 tiles: 512 threads 92 us, 1024 84; 3072 tiles 85 and 93)
         const int smem = cs_scatter_smem_bytes(T);
         const int threads = T <= 4096 ? 512 : 1024;
+        // The limit belongs to the function, for every thread and captured launch: always the largest
+        // grid's, so that no call lowers it under another's launch.
         if (smem + kScatterStatic > 48 * 1024)
-            GSV_CUDA_TRY(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            GSV_CUDA_TRY(cudaFuncSetAttribute(k_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              cs_scatter_smem_bytes(kCsMaxTiles)));
         k_scatter<<<unsigned(rows), threads, smem, st>>>(at<int32_t>(ws_gauss, G.cs_pos), at<int4>(ws_gauss, G.box),
                                                          offsets, n, int(row_len), T, s, cap, vals_out, status, lb_cs,
                                                          cs_col_blocks(T));
