@@ -148,8 +148,10 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                  : "memory");
 }
 
+// tcgen05.ld and its wait need the whole warp converged, wherever its lanes come from.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     uint32_t r[16];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
@@ -192,6 +194,7 @@ __device__ __forceinline__ float2 gelu_grad(float2 x) {
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
     uint32_t r[32];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
         "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -376,8 +379,7 @@ struct Chunk {
     __device__ static __forceinline__ void put(unsigned char* scr, uint32_t taddr, int lane) {
         float v[CW];
         if constexpr (CW == 32) tmem_ld32(taddr, v);
-        else tmem_ld16(taddr, v);
-        __syncwarp();  // the previous chunk has been read
+        else tmem_ld16(taddr, v);  // either begins with a __syncwarp: the previous chunk has been read
 #pragma unroll
         for (int p = 0; p < CW / 4; ++p)
             *reinterpret_cast<float4*>(scr + at(lane, p)) = make_float4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
@@ -414,9 +416,10 @@ __device__ __noinline__ void store_chunk(const GemmArgs& g, uint32_t taddr, unsi
                 for (int k = 0; k < 16; ++k) z[k] = g.z_f32[at + k * g.c_sn];
             }
             tmem_ld16(taddr + h, v);
-            if (!row_ok) continue;
+            if (row_ok) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) epi_store<EPI>(g, at + k * g.c_sn, v[k], bias_of(g, n0 + h + k), z[k]);
+                for (int k = 0; k < 16; ++k) epi_store<EPI>(g, at + k * g.c_sn, v[k], bias_of(g, n0 + h + k), z[k]);
+            }
         }
         return;
     }
