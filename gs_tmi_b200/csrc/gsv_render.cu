@@ -404,6 +404,21 @@ __device__ __forceinline__ bool needs_guard(const Rec& r) {
              fabsf(r.c2) <= kBig);
 }
 
+// A lane's moments: the packed loop's, or the guarded one's where the tile's gradient (`guard`) or the lane's
+// own Gaussian needs it.  The two round differently, so each lane keeps to its own: which Gaussians share
+// a warp depends on the cull and the execution shape, and must not show in their gradients.
+__device__ __forceinline__ void moments_of(const Rec& g, const float* gs, float v0, float v1, float v2, bool guard,
+                                           float m[kMomStride]) {
+    const bool wild = guard || needs_guard(g);
+    if (!guard) block_moments(g, gs, v0, v1, v2, m);
+    if (__any_sync(kFull, wild)) {
+        float mg[kMomStride];
+        block_moments_guarded(g, gs, v0, v1, v2, mg);
+#pragma unroll
+        for (int i = 0; i < kMomStride; ++i) m[i] = wild ? mg[i] : m[i];
+    }
+}
+
 // The moments of one (tile, Gaussian) pair to the gradients of the reference's own parameters.
 __device__ __forceinline__ void compat_emit_lane(const RenderArgs& a, const Rec& g, int gid, const float m[kMomStride],
                                                  const float ih[3]) {
@@ -782,14 +797,7 @@ __device__ __forceinline__ void backward_tile(const RenderArgs& a, int64_t tile,
             const float v0 = float(d0 + (b >> 2) * kBlk), v1 = float(h0 + ((b >> 1) & 1) * kBlk),
                         v2 = float(w0 + (b & 1) * kBlk);
             float m[kMomStride];
-            if (guard || __any_sync(kFull, needs_guard(g))) {
-                float mg[kMomStride];
-                block_moments_guarded(g, gs, v0, v1, v2, mg);
-#pragma unroll
-                for (int i = 0; i < kMomStride; ++i) m[i] = mg[i];
-            } else {
-                block_moments(g, gs, v0, v1, v2, m);
-            }
+            moments_of(g, gs, v0, v1, v2, guard, m);
             // a Gaussian may have two of its blocks among these lanes: one block at a time
             const int b_end = __shfl_sync(kFull, b, 31);
             for (int bb = __shfl_sync(kFull, b, 0); bb <= b_end; ++bb) {
@@ -1014,14 +1022,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_backward4(const RenderArgs a) {
         const Rec g = rec_of(S.rec[at][0], S.rec[at][1], S.rec[at][2]);
         const int gid = S.gid[at];
         float m[kMomStride];
-        if (guard || __any_sync(kFull, needs_guard(g))) {
-            float mg[kMomStride];
-            block_moments_guarded(g, S.grad, v0, v1, v2, mg);
-#pragma unroll
-            for (int i = 0; i < kMomStride; ++i) m[i] = mg[i];
-        } else {
-            block_moments(g, S.grad, v0, v1, v2, m);
-        }
+        moments_of(g, S.grad, v0, v1, v2, guard, m);
         if (on && !(DET && S.pidx[at] < 0)) {
             if (COMPAT) {
                 compat_emit_lane(a, g, gid, m, ih);
