@@ -467,9 +467,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_prepare(const float* __restric
         R.q00 = qc[0]; R.q01x2 = qc[1]; R.q02x2 = qc[2]; R.q11 = qc[3]; R.q12x2 = qc[4]; R.q22 = qc[5];
         R.rho_r = dr[g * dstride]; R.rho_i = di[g * dstride]; R.pad = 0.0f;
         recs[g] = R;
-        float4 x = tight_extent(qc);
-        x.w = plane_threshold(R);
-        ext[g] = x;
+        ext[g] = tight_extent(qc);
         cnt = tile_box(s, c, r, &box);
         if (cnt <= 0) {
             atomicOr(&status->flags, GSV_FLAG_EMPTY_BOX);

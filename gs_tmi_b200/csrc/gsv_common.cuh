@@ -105,7 +105,24 @@ __device__ __forceinline__ void qcoef_from_covinv(const float* m9, const float i
     }
 }
 
-// Conservative tight extent of the inclusion set {e : m_fp32(e) <= 9}.
+// Threshold of the separating-plane test of a block (plane_separates in gsv_render.cu) for a quadratic form
+// with anisotropy K = max_a Q_aa S_aa, S = Q^-1; infinity: nothing is separated.  The test runs in FP32 on
+// the stored coefficients, with u = 2^-24 and s = sum_a sqrt(Q_aa): its m is off by at most 8 u 9 K m
+// (4.3e-6 K m), its t by that and 1.1e-6 s sqrt(K m) (the rounding of n = Q e, |Q_ab e_b| <=
+// sqrt(Q_aa) sqrt(K m)), and the row form includes up to m = 9 (1 + 3.3e-6 K).  With twice each of these
+//   (3 sqrt(1 + 6.6e-6 K) + 2.2e-6 s sqrt(K))^2 / (1 - 8.6e-6 K)
+// is 9.31 at K = 1000, s = 400 and 11.1 at K = 1e4, s = 400, and the test's factor of m (plane_factor) times
+// 1 + 8.6e-6 K is below 1.  At K = 250, s = 800 single errors give 9.10, and the factor 0.99 leaves another
+// 0.026 sqrt(m), as much again.
+constexpr float kPlane250 = 9.1f, kPlane1000 = 9.35f, kPlane10000 = 11.2f;
+__device__ __forceinline__ float plane_factor(float thr) { return thr < 10.0f ? 0.99f : 0.9f; }
+__device__ __forceinline__ float plane_by_k(double k, float qmax) {  // k <= 1e4
+    if (k <= 250.0 && qmax < 7e4f) return kPlane250;
+    return qmax < 1.7e4f ? (k <= 1000.0 ? kPlane1000 : kPlane10000) : __int_as_float(0x7f800000);
+}
+
+// Conservative tight extent of the inclusion set {e : m_fp32(e) <= 9}, and in w the threshold of its
+// separating planes.
 //
 // For the exact quadratic form of the stored FP32 coefficients, m(e) <= 9
 // implies |e_a| <= 3 sqrt(S_aa) with S = Q^-1 (Schur complement bound).  The
@@ -115,7 +132,7 @@ __device__ __forceinline__ void qcoef_from_covinv(const float* m9, const float i
 // m <= 9 (1 + 3.3e-6 K).  The extent is widened by a factor
 // sqrt(1 + 1e-4 K) (30x that bound) plus 0.01 voxel for the FP32 rounding
 // of c -/+ extent at the culling site.  Q not positive definite, NaN, or
-// K > 1e4: infinite extent (nothing is culled).  Computed in FP64 from the
+// K > 1e4: infinite extent and threshold (nothing is culled).  Computed in FP64 from the
 // stored coefficients, rounded up.
 __device__ __forceinline__ float4 tight_extent(const float qc[6]) {
     const double q00 = qc[0], q01 = 0.5 * double(qc[1]), q02 = 0.5 * double(qc[2]);
@@ -124,31 +141,41 @@ __device__ __forceinline__ float4 tight_extent(const float qc[6]) {
     const double c01 = q02 * q12 - q01 * q22, c02 = q01 * q12 - q02 * q11;
     const double det = q00 * c00 + q01 * c01 + q02 * c02;
     const float inf = __int_as_float(0x7f800000);
-    if (!(q00 > 0.0 && c22 > 0.0 && det > 0.0 && c00 > 0.0 && c11 > 0.0)) return make_float4(inf, inf, inf, 0.f);
+    if (!(q00 > 0.0 && c22 > 0.0 && det > 0.0 && c00 > 0.0 && c11 > 0.0)) return make_float4(inf, inf, inf, inf);
     const double s0 = c00 / det, s1 = c11 / det, s2 = c22 / det;
     double k = q00 * s0;
     k = fmax(k, q11 * s1);
     k = fmax(k, q22 * s2);
-    if (!(k <= 1e4)) return make_float4(inf, inf, inf, 0.f);
+    if (!(k <= 1e4)) return make_float4(inf, inf, inf, inf);
     const double f = 9.0 * (1.0 + 1e-4 * k);
     return make_float4(__double2float_ru(sqrt(f * s0) + 0.01), __double2float_ru(sqrt(f * s1) + 0.01),
-                       __double2float_ru(sqrt(f * s2) + 0.01), 0.f);
+                       __double2float_ru(sqrt(f * s2) + 0.01), plane_by_k(k, fmaxf(qc[0], fmaxf(qc[3], qc[5]))));
 }
 
-// Threshold of the separating-plane test of a block (plane_separates in gsv_render.cu): 9.1, or
-// infinity (nothing is separated) where rounding could decide it.  The test is run in FP32 on the
-// stored coefficients; with K = max_a Q_aa S_aa <= 250 and sum_a sqrt(Q_aa) <= 800 its relative
-// errors stay below 2e-3 (m) and 0.014 sqrt(m) (t), and the row form's m is within 8.3e-4 of the exact
-// one: 0.99, 1.515 and 9.1 leave at least as much again.  K <= 1 / det(C) for the correlation matrix C of Q
-// (a cofactor of C is at most 1), and det(C) is computed here to about 1e-6.
+// The reference-signature kernels cull by planes alone, whose threshold (plane_by_k) is found for each
+// listed pair.  Most Gaussians are told in FP32: K <= 1 / det(C), C the correlation matrix of Q (a cofactor of
+// C is at most 1), and det(C) = det(Q) / (q00 q11 q22) comes out to about 1e-6, so 1 / 250 is far from its
+// rounding (and an indefinite Q from passing); coefficients above 1e-10 keep the products from underflowing.
+// The rest in FP64: K <= b as max_a Q_aa c_aa <= b det(Q), c the cofactors.  Neither divides: three
+// reciprocals, or FP64 for all, cost a forward of round Gaussians up to 3 us in 34.  Without the second part
+// flat sets lose the cull; 100x84x60, 20k needles of 33 : 1 over 332 tiles each, forward 1330 -> 217 us and
+// backward 2020 -> 208; 20k pancakes of 15 : 1, 493 -> 173 and 717 -> 219.
 __device__ __forceinline__ float plane_threshold(const Rec& r) {
     const float h01 = 0.5f * r.q01x2, h02 = 0.5f * r.q02x2, h12 = 0.5f * r.q12x2;
-    const float i0 = 1.0f / r.q00, i1 = 1.0f / r.q11, i2 = 1.0f / r.q22;
-    const float r01 = h01 * h01 * i0 * i1, r02 = h02 * h02 * i0 * i2, r12 = h12 * h12 * i1 * i2;
-    const float det = 1.0f + 2.0f * (h01 * i0) * (h02 * i2) * (h12 * i1) - r01 - r02 - r12;
-    const bool ok = r.q00 > 0.0f && r.q11 > 0.0f && r.q22 > 0.0f && r.q00 < 7e4f && r.q11 < 7e4f && r.q22 < 7e4f &&
-                    r01 < 1.0f && r02 < 1.0f && r12 < 1.0f && det >= 1.0f / 250.0f;
-    return ok ? 9.1f : __int_as_float(0x7f800000);
+    const float qmax = fmaxf(fmaxf(r.q00, r.q11), r.q22);
+    {
+        const float c00 = r.q11 * r.q22 - h12 * h12, c11 = r.q00 * r.q22 - h02 * h02, c22 = r.q00 * r.q11 - h01 * h01;
+        const float det = r.q00 * c00 + h01 * (h02 * h12 - h01 * r.q22) + h02 * (h01 * h12 - h02 * r.q11);
+        if (fminf(fminf(r.q00, r.q11), r.q22) > 1e-10f && qmax < 7e4f && c00 > 0.0f && c11 > 0.0f && c22 > 0.0f &&
+            250.0f * det >= r.q00 * r.q11 * r.q22)
+            return kPlane250;
+    }
+    const double q00 = r.q00, q01 = h01, q02 = h02, q11 = r.q11, q12 = h12, q22 = r.q22;
+    const double c00 = q11 * q22 - q12 * q12, c11 = q00 * q22 - q02 * q02, c22 = q00 * q11 - q01 * q01;
+    const double det = q00 * c00 + q01 * (q02 * q12 - q01 * q22) + q02 * (q01 * q12 - q02 * q11);
+    const double top = fmax(q00 * c00, fmax(q11 * c11, q22 * c22));
+    if (!(q00 > 0.0 && c22 > 0.0 && det > 0.0 && c00 > 0.0 && c11 > 0.0 && top <= 1e4 * det)) return __int_as_float(0x7f800000);
+    return plane_by_k(top <= 250.0 * det ? 250.0 : (top <= 1000.0 * det ? 1000.0 : 1e4), qmax);
 }
 
 // Row terms of the quadratic form for fixed (e0, e1):

@@ -239,12 +239,13 @@ __device__ __forceinline__ Rec rec_of(float4 x, float4 y, float4 z) {
 
 // Separating plane of a Gaussian's inclusion set and a block, from the block centre's offset e to the
 // Gaussian: with n = Q e (the gradient there, up to a factor), the block's voxels x satisfy
-// n.x >= m(e) - 1.5 |n|_1, and {m <= 9} lies in n.x <= 3 sqrt(m(e)).  `thr`: plane_threshold.  On
+// n.x >= m(e) - 1.5 |n|_1, and {m <= 9} lies in n.x <= 3 sqrt(m(e)).  `thr`: plane_by_k.  On
 // fits' Gaussians 93-96% of the blocks kept by this test and the extent hold an included voxel;
 // the extent's box alone keeps 1.4 to 1.6 times as many.
-__device__ __forceinline__ bool plane_separates(float n0, float n1, float n2, float e0, float e1, float e2, float thr) {
+__device__ __forceinline__ bool plane_separates(float n0, float n1, float n2, float e0, float e1, float e2, float thr,
+                                                float factor) {
     const float m = fmaf(n0, e0, fmaf(n1, e1, n2 * e2));
-    const float t = fmaf(-1.515f, fabsf(n0) + fabsf(n1) + fabsf(n2), 0.99f * m);
+    const float t = fmaf(-1.515f, fabsf(n0) + fabsf(n1) + fabsf(n2), factor * m);
     return t > 0.0f && t * t > thr * m;
 }
 
@@ -263,7 +264,7 @@ __device__ __forceinline__ unsigned block_mask8(const Rec& r, float4 x, int d0, 
         in &= ((lo2 <= float(w0 + 3) && hi2 >= float(w0)) ? 0x55u : 0u) |
               ((lo2 <= float(w0 + 7) && hi2 >= float(w0 + 4)) ? 0xaau : 0u);
     }
-    const float thr = x.w;
+    const float thr = x.w, factor = plane_factor(thr);
     const float h01 = 0.5f * r.q01x2, h02 = 0.5f * r.q02x2, h12 = 0.5f * r.q12x2;
 #pragma unroll
     for (int bd = 0; bd < 2; ++bd) {
@@ -275,7 +276,7 @@ __device__ __forceinline__ unsigned block_mask8(const Rec& r, float4 x, int d0, 
 #pragma unroll
             for (int bw = 0; bw < 2; ++bw) {
                 const float e2 = float(w0 + 4 * bw) + 1.5f - r.c2;
-                if (plane_separates(fmaf(h02, e2, a0), fmaf(h12, e2, a1), fmaf(r.q22, e2, a2), e0, e1, e2, thr))
+                if (plane_separates(fmaf(h02, e2, a0), fmaf(h12, e2, a1), fmaf(r.q22, e2, a2), e0, e1, e2, thr, factor))
                     in &= ~(1u << (4 * bd + 2 * bh + bw));
             }
         }
@@ -865,7 +866,7 @@ __device__ __forceinline__ bool block_hit(const Rec& r, float4 x, int d0, int h0
     const float h01 = 0.5f * r.q01x2, h02 = 0.5f * r.q02x2, h12 = 0.5f * r.q12x2;
     const float e0 = float(d0) + 1.5f - r.c0, e1 = float(h0) + 1.5f - r.c1, e2 = float(w0) + 1.5f - r.c2;
     return !plane_separates(fmaf(r.q00, e0, fmaf(h01, e1, h02 * e2)), fmaf(h01, e0, fmaf(r.q11, e1, h12 * e2)),
-                            fmaf(h02, e0, fmaf(h12, e1, r.q22 * e2)), e0, e1, e2, x.w);
+                            fmaf(h02, e0, fmaf(h12, e1, r.q22 * e2)), e0, e1, e2, x.w, plane_factor(x.w));
 }
 
 // A listed Gaussian of a 4^3 tile and whether its block is kept.
