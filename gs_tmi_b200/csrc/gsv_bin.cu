@@ -59,10 +59,10 @@ int sort_end_bit(int64_t ntiles) {
 constexpr int kPrepThreads = 256;
 __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPrepThreads - 1) / kPrepThreads; }
 
-// Counting-sort binning, used unless the tile grid is very large.  The pairs'
+// Counting-sort binning, used unless the tile grid is large for the pairs (cs_pays).  The pairs'
 // final order is fixed by two facts: a tile's list holds its Gaussians in
 // ascending id, and Gaussians are handled in rows of consecutive ids.  The
-// kernel that counts the pairs also writes, per row, how many of the row's
+// kernel that counts the pairs, or k_count_rows, also writes, per row, how many of the row's
 // pairs fall in each tile (rows x tiles 16-bit counts, "cs_mat", rows padded
 // to whole words); k_colscan writes, per row and tile, the position of the
 // row's first pair of that tile in the sorted output ("cs_pos": the column's
@@ -115,6 +115,31 @@ inline bool cs_eligible(int64_t n, int64_t ntiles) {
     return n > 0 && ntiles <= kCsMaxTiles &&
            cs_rows(n, ntiles) * ntiles <= (ntiles <= kCsSmallTiles ? 2 * kCsMaxCells : kCsMaxCells);
 }
+// Up to kCsSmallTiles tiles the counting sort is the faster one from 50 Gaussians to a million.  On larger grids
+// its row counts have to pay: their filling and scanning grow with rows x tiles (7 us a million), the radix sort
+// with the pairs (20 us a million more than 50, where one block cannot sort them; its buffers are the
+// capacity's size).  Where the Gaussians alone decide for the counting sort (each has a pair at least), the
+// kernel that counts a Gaussian's pairs fills its rows of cs_mat at once; elsewhere gsv_bin decides, and only
+// then are the rows counted, by a kernel of their own (3 us).  Preprocess and binning, us:
+//   tiles  Gaussians  row counts    pairs   counting   radix
+//    3456        50     0.003 M       163     18.8      16.5
+//   18432       500     0.04 M      1,551     33.7      18.2
+//    3456     2,000     0.03 M      6,199     25.0      48.8
+//   18432     5,000     0.4 M      15,967     36.7      50.4
+//    9120   100,000     3.6 M     320,000     54.1      58.8
+//    4096   300,000     4.8 M     946,000     72.9      79.5
+//   13824   100,000     5.4 M     319,000     73.5      57.9
+//   18432   100,000     7.2 M     320,000     83.9      56.9
+//    6000   300,000     7.0 M     948,000     93.8      77.5
+//   13824   100,000     5.4 M   2,440,000      101      95.4
+//   18432   100,000     7.2 M   2,460,000      116      97.7
+//    9216   154,793     5.6 M   5,570,000      130       159
+constexpr int64_t kCsFewPairs = 4096, kCsFreeCells = 3900000;
+inline int64_t cs_cells(int64_t n, int64_t ntiles) { return cs_rows(n, ntiles) * ntiles; }
+inline bool cs_pays(int64_t n, int64_t ntiles, int64_t pairs) {
+    return ntiles <= kCsSmallTiles || (pairs > kCsFewPairs && cs_cells(n, ntiles) < kCsFreeCells + pairs);
+}
+inline bool cs_fused(int64_t n, int64_t ntiles) { return cs_pays(n, ntiles, n); }
 
 // Status region: the Status word, the preprocess's look-back words (one per
 // block), then k_colscan's (one per column block).  Status::pad[1] and
@@ -504,6 +529,20 @@ __global__ void __launch_bounds__(kPrepThreads) k_count_compat(const float* __re
     if (cs_mat != nullptr) count_rows(s, box, sc, bid, row_len, cs_mat, ntiles);  // block-uniform
 }
 
+// count_rows from the tile boxes of an earlier launch (where not cs_fused).
+__global__ void __launch_bounds__(kPrepThreads) k_count_rows(const int4* __restrict__ boxes, int64_t n, DevShape s,
+                                                             uint16_t* __restrict__ cs_mat, int32_t row_len, int32_t ntiles) {
+    const int64_t bid = blockIdx.x, g = bid * kPrepThreads + threadIdx.x;
+    const int4 box = g < n ? boxes[g] : make_int4(0, 0, 0, 0);
+    int64_t incl = box.w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((threadIdx.x & 31) >= o) incl += y;
+    }
+    count_rows(s, box, PairScan{incl - box.w, __shfl_sync(0xffffffffu, incl, 31)}, bid, row_len, cs_mat, ntiles);
+}
+
 // Emission of the pairs in Gaussian-major (d,h,w) raster order
 // (tile_voxelizer.py:126-145), plus the two fills the sort and the range
 // pass need: the tile ranges cleared to (0,0) and the sort padding past the
@@ -817,10 +856,15 @@ int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, s
         GSV_CUDA_TRY(cudaMemsetAsync(ranges, 0, size_t(si.ntiles) * sizeof(int2), st));
         return GSV_OK;
     }
-    if (G.cs && mode != GSV_BIN_RADIX) {
+    if (G.cs && (mode == GSV_BIN_COUNTING || (mode == GSV_BIN_AUTO && cs_pays(n, si.ntiles, cap)))) {
         unsigned long long* lb_cs = reinterpret_cast<unsigned long long*>(status + 1) + prep_blocks(n);
         const int64_t rows = cs_rows(n, si.ntiles), row_len = cs_row_len(n, si.ntiles);
         const int32_t T = int32_t(si.ntiles);
+        if (!cs_fused(n, T)) {
+            k_count_rows<<<unsigned(prep_blocks(n)), kPrepThreads, cs_count_smem_bytes(n, T), st>>>(
+                at<int4>(ws_gauss, G.box), n, s, at<uint16_t>(ws_gauss, G.cs_mat), int32_t(row_len), T);
+            GSV_LAUNCH_CHECK();
+        }
         k_colscan<<<unsigned(cs_col_blocks(T)), kCsCols * kCsRowGroups, 0, st>>>(
             at<uint16_t>(ws_gauss, G.cs_mat), at<int32_t>(ws_gauss, G.cs_pos), rows, T, cap, ranges, status, lb_cs);
         GSV_LAUNCH_CHECK();
@@ -916,11 +960,12 @@ static int prepare_impl(const gsv_params* p, int64_t density_stride, const int32
     Status* status = at<Status>(ws_gauss, L.status);
     // status flags, the block counters and the scans' look-back words
     GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
-    const int smem = L.cs ? cs_count_smem_bytes(n, si.ntiles) : 0;
+    const bool count = L.cs && cs_fused(n, si.ntiles);
+    const int smem = count ? cs_count_smem_bytes(n, si.ntiles) : 0;
     k_prepare<<<unsigned(prep_blocks(n)), kPrepThreads, smem, st>>>(
         p->positions, p->scales, p->rotations, p->density_r, p->density_i, density_stride, n, live, dev_shape(si),
         at<Rec>(ws_gauss, L.rec), at<float4>(ws_gauss, L.ext), at<int4>(ws_gauss, L.box),
-        at<int64_t>(ws_gauss, L.offsets), status, L.cs ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr,
+        at<int64_t>(ws_gauss, L.offsets), status, count ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr,
         int32_t(cs_row_len(n, si.ntiles)), int32_t(si.ntiles), at<float>(ws_gauss, L.accum));
     GSV_LAUNCH_CHECK();
     if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, flags_host, st);
@@ -995,9 +1040,10 @@ int gsv_build_tile_pairs_count(const float* center_vox, const float* radius_vox,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Status* status = at<Status>(ws_gauss, L.status);
     GSV_CUDA_TRY(cudaMemsetAsync(status, 0, status_bytes(n, si.ntiles), st));
-    k_count_compat<<<unsigned(prep_blocks(n)), kPrepThreads, L.cs ? cs_count_smem_bytes(n, si.ntiles) : 0, st>>>(
+    const bool count = L.cs && cs_fused(n, si.ntiles);
+    k_count_compat<<<unsigned(prep_blocks(n)), kPrepThreads, count ? cs_count_smem_bytes(n, si.ntiles) : 0, st>>>(
         center_vox, radius_vox, n, dev_shape(si), at<int4>(ws_gauss, L.box), at<int64_t>(ws_gauss, L.offsets), status,
-        L.cs ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr, int32_t(cs_row_len(n, si.ntiles)), int32_t(si.ntiles));
+        count ? at<uint16_t>(ws_gauss, L.cs_mat) : nullptr, int32_t(cs_row_len(n, si.ntiles)), int32_t(si.ntiles));
     GSV_LAUNCH_CHECK();
     if (total_pairs_host) return read_status(L, ws_gauss, total_pairs_host, nullptr, st);
     return GSV_OK;

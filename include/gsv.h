@@ -141,12 +141,14 @@ GSV_API int gsv_prepare_strided(const gsv_params* params, int64_t density_stride
  * `capacity` pairs are kept and GSV_FLAG_CAPACITY_OVERFLOW is latched.  May
  * be called again after one preprocess (e.g. with a larger capacity).
  * Two sorts give the same lists: a counting sort over per-row tile counts
- * the preprocess writes when the grid has at most 18432 tiles and
- * ceil((n+1)/256) x tiles <= 2^23, or 2^24 on at most 3072 tiles (three launches, no pair keys), else an emit + radix sort + range pass.  gsv_bin picks the first
- * where it applies. */
+ * (no pair keys), for grids of at most 18432 tiles with
+ * ceil((n+1)/256) x tiles <= 2^23, or 2^24 on at most 3072 tiles, and an
+ * emit + radix sort + range pass.  gsv_bin takes the first where it applies
+ * and is the faster: on at most 3072 tiles always, on more where `capacity`
+ * is above 4096 and ceil((n+1)/256) x tiles below 3.9 million + capacity. */
 #define GSV_BIN_AUTO 0
 #define GSV_BIN_RADIX 1    /* always the radix sort */
-#define GSV_BIN_COUNTING 2 /* the counting sort; GSV_ERR_INVALID_ARGUMENT where it does not apply */
+#define GSV_BIN_COUNTING 2 /* always the counting sort; GSV_ERR_INVALID_ARGUMENT where it does not apply */
 GSV_API int gsv_bin(gsv_shape shape, int64_t n, void* ws_gauss, void* ws_pairs, size_t ws_pairs_bytes,
             int64_t capacity, void* stream);
 GSV_API int gsv_bin_ex(gsv_shape shape, int64_t n, void* ws_gauss, void* ws_pairs, size_t ws_pairs_bytes,
