@@ -13,13 +13,15 @@ Two knobs change speed but not results (every candidate evaluates the same
 
 ``Autotuner.pick`` times every candidate's forward + backward on the binned
 problem at hand with CUDA events and keeps the fastest, cached per
-(volume shape, Gaussian-count bucket, backward mode); the cache can be
-persisted as JSON.  The deterministic backward always runs whole tiles, so
+(volume shape, Gaussian-count bucket, backward mode) and build of the
+kernels; the cache can be persisted as JSON.  The deterministic backward always runs whole tiles, so
 only the forward takes the half-tile shape there.
 """
 from __future__ import annotations
 
 import ctypes
+import functools
+import hashlib
 import json
 import math
 import os
@@ -28,7 +30,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
-from ._lib import GsvGrads, GsvParams, GsvTuning, check, lib
+from ._lib import LIB_PATH, GsvGrads, GsvParams, GsvTuning, check, lib
 
 # (rows per lane, Gaussian batch[, backward list split])
 CANDIDATES: Tuple[Tuple[int, ...], ...] = ((2, 32), (2, 16), (1, 32), (1, 16), (1, 8), (2, 32, 2), (1, 32, 2),
@@ -44,6 +46,13 @@ def tuning_of(c) -> GsvTuning:
 
 def label_of(c) -> str:
     return "/".join(str(int(x)) for x in c) if len(c) > 2 and int(c[2]) > 1 else f"{int(c[0])}/{int(c[1])}"
+
+
+@functools.lru_cache(maxsize=None)
+def kernels_id() -> str:
+    """The kernels' build, by the library's content: a saved pick that was measured on others is not used."""
+    with open(LIB_PATH, "rb") as f:
+        return hashlib.sha256(f.read()).hexdigest()[:12]
 
 
 def _ptr(t):
@@ -64,7 +73,14 @@ class Autotuner:
     @staticmethod
     def key(shape, n: int, deterministic: bool) -> str:
         b = int(math.ceil(math.log2(max(n, 1))))
-        return f"{shape.d}x{shape.h}x{shape.w}/ts{shape.tile_size}/n2^{b}/{'det' if deterministic else 'atomic'}"
+        mode = "det" if deterministic else "atomic"
+        return f"{kernels_id()}/{shape.d}x{shape.h}x{shape.w}/ts{shape.tile_size}/n2^{b}/{mode}"
+
+    @staticmethod
+    def tile_key(volume_shape, n: int, deterministic: bool) -> str:
+        d, h, w = (int(x) for x in volume_shape)
+        mode = "det" if deterministic else "atomic"
+        return f"{kernels_id()}/{d}x{h}x{w}/n2^{int(math.ceil(math.log2(max(n, 1))))}/{mode}/tile"
 
     def save(self):
         if self.path:
@@ -133,7 +149,7 @@ class Autotuner:
 
         n = int(params[0].shape[0])
         d, h, w = (int(x) for x in volume_shape)
-        k = f"{d}x{h}x{w}/n2^{int(math.ceil(math.log2(max(n, 1))))}/{'det' if flags & 1 else 'atomic'}/tile"
+        k = self.tile_key(volume_shape, n, bool(flags & 1))
         with self._lock:
             if k in self.cache:
                 ts, *shape_t = self.cache[k]
