@@ -1712,8 +1712,10 @@ int gsv_backward_strided(const gsv_params* p, gsv_shape shape, void* ws_gauss, v
     a.prm = *p;
     a.grd = *grads;
     a.dstride = density_stride;
-    // four Gaussians a warp while the warps are few, 32 (every lane busy in the chain rule) above
-    if (det && capacity > 0 && n < 131072) k_finalize_det<1><<<grid_for(n, 32), 256, 0, st>>>(a);
+    // Four Gaussians a warp while the warps are few, 32 (every lane busy in the chain rule) above.  Whole
+    // backward with 4 and 32, 11 pairs a Gaussian, us: 30,000 65 and 70; 48,000 84 and 86; 56,000 91 and 91;
+    // 65,000 101 and 98; 131,000 189 and 179; 400,000 369 and 320; the same within 1% on other grids.
+    if (det && capacity > 0 && n < 57344) k_finalize_det<1><<<grid_for(n, 32), 256, 0, st>>>(a);
     else if (det && capacity > 0) k_finalize_det<8><<<grid_for(n, 256), 256, 0, st>>>(a);
     else k_finalize<<<grid_for(n, 256), 256, 0, st>>>(a);
     GSV_LAUNCH_CHECK();
