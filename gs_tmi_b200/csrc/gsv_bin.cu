@@ -391,7 +391,11 @@ __device__ __forceinline__ PairScan scan_counts(int64_t cnt, int64_t n, int64_t 
 // stride over its pairs, the block-local range [o of lane 0, warp_end), lane l's
 // Gaussian the part starting at o, and find each pair's Gaussian by a shuffle
 // search over the 32 starts (zero-count lanes share their successor's start
-// and are never chosen).
+// and are never chosen).  The first costs little more with more pairs, the second a search for each: they cross
+// at 16 pairs a Gaussian.  k_prepare, first and second way, us: 20,000 Gaussians with 6 pairs 16.3 and
+// 13.5, 15 pairs 16.1 and 16.1, 24 pairs 16.6 and 19.0; 100,000 with 11 pairs 25.0 and 22.8, 16 pairs 24.7
+// and 24.5, 18 pairs 25.3 and 25.9, 27 pairs 26.2 and 29.7.
+constexpr int kCountWide = 16;
 __device__ __forceinline__ void count_rows(const DevShape& s, int4 box, const PairScan& sc, int64_t bid, int row_len,
                                            uint16_t* __restrict__ cs_mat, int32_t ntiles) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -406,7 +410,7 @@ __device__ __forceinline__ void count_rows(const DevShape& s, int4 box, const Pa
     const long long wstart = __shfl_sync(kAll, o, 0);
     const long long wend = sc.warp_end;
     const float rcp1 = box_rcp(box.z), rcp2 = box_rcp(box.z >> 16);
-    if (wend - wstart >= 32 * 24) {
+    if (wend - wstart >= 32 * kCountWide) {
         for (int j = 0; j < 32; ++j) {
             const int cnt = __shfl_sync(kAll, box.w, j);
             const int bx = __shfl_sync(kAll, box.x, j), by = __shfl_sync(kAll, box.y, j), bz = __shfl_sync(kAll, box.z, j);
@@ -868,8 +872,11 @@ int bin_common(const ShapeInfo& si, int64_t n, void* ws_gauss, void* ws_pairs, s
         k_colscan<<<unsigned(cs_col_blocks(T)), kCsCols * kCsRowGroups, 0, st>>>(
             at<uint16_t>(ws_gauss, G.cs_mat), at<int32_t>(ws_gauss, G.cs_pos), rows, T, cap, ranges, status, lb_cs);
         GSV_LAUNCH_CHECK();
-        // a long row over many tiles is a chain of long sub-rows, one block to an SM: more threads shorten
-        // them (13824 tiles: 512 threads 92 us, 1024 84; 3072 tiles 85 and 93)
+        // Short rows of many blocks take 512 threads, with which more blocks fit on an SM; more threads shorten the
+        // sweeps over many tiles, of which one block fits from 9088 on.  Binning with 512 and 1024, us: 3072 tiles,
+        // 50,000 Gaussians 22 and 25, 200,000 42 and 48; 4096 tiles 26 and 26, 45 and 51; 8832 tiles, 20,000 36 and
+        // 34, 100,000 49 and 47; 9384 tiles 37 and 33, 61 and 52; 17576 tiles 51 and 44, 103 and 90.  Between 4096
+        // and 9088 either may be the faster: 5760 tiles, 200,000 75 and 81; 6336 tiles, 100,000 44 and 42.
         const int smem = cs_scatter_smem_bytes(T);
         const int threads = T <= 4096 ? 512 : 1024;
         // The limit belongs to the function, for every thread and captured launch: always the largest
