@@ -1697,7 +1697,7 @@ int gsv_backward_strided(const gsv_params* p, gsv_shape shape, void* ws_gauss, v
     if (tuning) {
         a.chunk = tuning->chunk;
         a.cull = !(tuning->flags & GSV_TUNE_NO_CULL);
-        a.split = tuning->split > 0 ? tuning->split : 1;
+        if (tuning->split > 0) a.split = tuning->split;
     }
     if (ntiles * 2 * a.split > int64_t(INT32_MAX)) return GSV_ERR_INVALID_ARGUMENT;
     const int rpl = (tuning && !det) ? tuning->rows_per_lane : 2;  // deterministic: whole tiles

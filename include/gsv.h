@@ -228,7 +228,7 @@ typedef struct gsv_tuning {
     int32_t chunk;
     int32_t flags;
     int32_t split; /* backward, tile edge 8: most CTAs sharing one (half) tile's Gaussian list, 1, 2 or 4
-                      (0 = 1; without a gsv_tuning it is chosen by the tile count) */
+                      (0 = chosen by the tile count) */
 } gsv_tuning;
 
 /* gsv_forward / gsv_backward with an explicit execution shape (NULL =
