@@ -293,6 +293,8 @@ def voxelize(positions: torch.Tensor, scales: torch.Tensor, rotations: torch.Ten
     """Functional form: complex64 (D,H,W) volume, differentiable in all five
     parameter tensors.  `tuner`: an autotune.Autotuner picking the execution
     shape (results do not depend on it)."""
+    if density_i is None:
+        raise TypeError("density_i must be a tensor (TileVoxelizer takes a complex density)")
     return _VoxelizeFn.apply(positions, scales, rotations, density_r, density_i,
                              _shape(volume_shape, tile_size), bool(deterministic), tuner)
 
