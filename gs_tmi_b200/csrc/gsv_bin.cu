@@ -74,19 +74,30 @@ __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPre
 //
 // A row is 64 Gaussians, which gives k_scatter many short blocks, while there
 // are no more rows than tiles (a column of k_colscan grows with the rows, a
-// block of k_scatter with the tiles) and few row counts; otherwise 256 (a block
-// of the counting kernel).  Preprocess and binning with rows of 64, of 256 and
-// the radix sort, us:
+// block of k_scatter with the tiles), few row counts and at most 4096 tiles (4845:
+// 50,000 Gaussians 52.1 and 49.6); otherwise 256 (a block of the counting kernel).
+// Preprocess and binning with rows of 64, of 256 and the radix sort, us:
 //   tiles  Gaussians (pairs each)   64    256   radix
 //     512    20,000 (15)           28.5   30.9   55.4
 //     512    60,000 (11)           40.3   37.3
 //     512   200,000 (6)            65.0   52.7   79.2
 //    1728   120,000 (15)           59.2   56.7
 //    3072    50,000 (36)           48.9   54.6   87.4
+//    3072    75,000 (11)           50.0   46.5
+//    3072    85,000 (11)           55.7   53.3
+//    3072    85,000 (38)           68.7   71.8
 //    3072   200,000 (16)           92.8   79.5  126
 //    3072   500,000 (10)          210    140    182
 //    3072   800,000 (8)                  198    228
 //    3072 1,300,000 (6)                  297    298
+//    3456     2,000 (11)           27.7   32.9
+//    3456    20,000 (38)           40.8   46.0
+//    3456    40,000 (77)           61.4   74.2
+//    3456    50,000 (12)           42.5   45.1
+//    3456    64,000 (12)           43.2   42.1
+//    3840    50,000 (39)           54.4   60.2
+//    4096    50,000 (39)           54.9   60.9
+//    4096    60,000 (39)           60.3   61.1
 //    9216   154,793 (36)                 130    159
 //    9216   400,000 (20)                 251    224
 //   13824    40,000 (139)                133    179
@@ -97,14 +108,15 @@ __host__ __device__ inline int64_t prep_blocks(int64_t n) { return (n + 1 + kPre
 // 16.3; 139 pairs 130, 95, 84.
 constexpr int64_t kCsNarrow8 = 12, kCsNarrow16 = 24;
 constexpr int kCsSub = 64;  // Gaussians k_scatter places at a time: a bit each in a tile's word
-constexpr int64_t kCsSmallTiles = 3072;                // 64-Gaussian rows up to here: four rows of counters
-constexpr int64_t kCsSmallCells = int64_t(1) << 22;    // ... and up to this many row counts
+constexpr int64_t kCsShortTiles = 4096;                // 64-Gaussian rows up to here: four rows of counters
+constexpr int64_t kCsShortCells = 3500000;             // ... and up to this many row counts
+constexpr int64_t kCsSmallTiles = 3072;                // up to here always the counting sort (cs_pays), with
 constexpr int64_t kCsMaxTiles = 18432;                 // 12 bytes per tile in k_scatter's shared memory (227 KB)
-constexpr int64_t kCsMaxCells = int64_t(1) << 23;      // 16 MB of counts, 32 MB of positions; on few tiles twice that
+constexpr int64_t kCsMaxCells = int64_t(1) << 23;      // ... twice these 16 MB of counts and 32 MB of positions
 constexpr int kCsCols = 32, kCsRowGroups = 32;         // k_colscan block: 32 columns x 32 row groups
 __host__ __device__ inline int64_t cs_row_len(int64_t n, int64_t ntiles) {
     const int64_t rows = prep_blocks(n) * (kPrepThreads / kCsSub);
-    return ntiles <= kCsSmallTiles && rows <= ntiles && rows * ntiles <= kCsSmallCells ? kCsSub : kPrepThreads;
+    return ntiles <= kCsShortTiles && rows <= ntiles && rows * ntiles <= kCsShortCells ? kCsSub : kPrepThreads;
 }
 __host__ __device__ inline int64_t cs_rows(int64_t n, int64_t ntiles) {
     return prep_blocks(n) * (kPrepThreads / cs_row_len(n, ntiles));
@@ -832,7 +844,7 @@ int cs_count_smem_bytes(int64_t n, int64_t ntiles) {
 }
 int cs_scatter_smem_bytes(int64_t ntiles) { return int(ntiles * int64_t(sizeof(uint2) + sizeof(int32_t))); }
 constexpr int kScatterStatic = kPrepThreads * int(sizeof(int4) + sizeof(float2));
-static_assert((kCsMaxTiles + 1) / 2 * 4 <= 40 * 1024 && kPrepThreads / kCsSub * (kCsSmallTiles + 1) / 2 * 4 <= 40 * 1024,
+static_assert((kCsMaxTiles + 1) / 2 * 4 <= 40 * 1024 && kPrepThreads / kCsSub * (kCsShortTiles + 1) / 2 * 4 <= 40 * 1024,
               "the row counters leave no room for the static words");
 static_assert(kCsMaxTiles * (sizeof(uint2) + sizeof(int32_t)) + kScatterStatic <= 227 * 1024,
               "k_scatter's words, positions and boxes exceed an SM's shared memory");
