@@ -1,4 +1,4 @@
-// gsv_bin.cu -- preprocess and tile binning (device radix sort), sm_100a.
+// gsv_bin.cu -- preprocess and tile binning (counting sort or device radix sort), sm_100a.
 //
 // Binning is bit-exact with build_tile_pairs (3DGS/3dgsVC/gaussian/
 // tile_voxelizer.py:87-162): the FP32 center/radius follow :284-286 op for
@@ -12,7 +12,6 @@
 
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 
 #include "gsv_common.cuh"
 
@@ -132,7 +131,7 @@ inline bool cs_eligible(int64_t n, int64_t ntiles) {
 // with the pairs (20 us a million more than 50, where one block cannot sort them; its buffers are the
 // capacity's size).  Where the Gaussians alone decide for the counting sort (each has a pair at least), the
 // kernel that counts a Gaussian's pairs fills its rows of cs_mat at once; elsewhere gsv_bin decides, and only
-// then are the rows counted, by a kernel of their own (3 us).  Preprocess and binning, us:
+// then are the rows counted, by a kernel of their own (3 us more).  Preprocess and binning, us:
 //   tiles  Gaussians  row counts    pairs   counting   radix
 //    3456        50     0.003 M       163     18.8      16.5
 //   18432       500     0.04 M      1,551     33.7      18.2

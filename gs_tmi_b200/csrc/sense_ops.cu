@@ -66,7 +66,7 @@ __device__ __forceinline__ void store_cx(float2* p, const Cx<N>& r) {
 // the mask and the index arithmetic are taken once for all coils.  Bound by memory; kUnroll coils' loads are
 // in flight together.  N = 2 needs rows of a multiple of four (their half shift is even) and 16-byte
 // aligned arrays.  128x128x96 with 8 coils, us, against a row of one coil per warp: expand 47 -> 32,
-// residual 78 -> 44, adjoint 40 -> 35 (201, 307 and 214 MB: 6.3 to 7 TB/s).
+// residual 78 -> 44, adjoint 40 -> 35 (214, 308 and 214 MB read and written: 6.7, 7.0 and 6.1 TB/s).
 constexpr int kUnroll = 4;
 
 // Voxel group x (of v / N, I: an index type that holds it): its element offset and that of the place
